@@ -17,18 +17,12 @@ A program loads its weights once and serves many requests, so the model (seeded 
 shape) is kept per process; prompts, given tokens and logits come from the seed, and each state has a KV cache of
 its own.
 """
-import os
-import sys
 import weakref
 
 import numpy as np
 import torch
 
-ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-if ROOT not in sys.path:
-    sys.path.insert(0, ROOT)
-
-from __graft_entry__ import load_package  # noqa: E402
+from __graft_entry__ import load_package
 
 REQUEST_SEQ = 4224   # cache rows of a request: a 4096-token prompt and 128 tokens
 BATCH_SEQ = 1536     # cache rows per sequence of a batch
