@@ -20,6 +20,7 @@ SOURCES = [
     "csrc/gemm_tc.cu",
     "csrc/gemm_smallm.cu",
     "csrc/prefill.cu",
+    "csrc/attn_prefill.cu",
     "csrc/sampler.cu",
     "csrc/tp_rows.cu",
     "host/model.cu",

@@ -291,6 +291,26 @@ int make_map(CUtensorMap *map, const void *base, int rows, int k, int box_rows) 
     return LLMB_OK;
 }
 
+int make_map_3d(CUtensorMap *map, const void *base, int d0, int d1, int d2, size_t stride1, size_t stride2, int box1, int box2) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) {
+        set_last_error("cuTensorMapEncodeTiled is not available from this driver");
+        return LLMB_ERR_UNSUPPORTED;
+    }
+    const cuuint64_t dims[3] = {(cuuint64_t)d0, (cuuint64_t)d1, (cuuint64_t)d2};
+    const cuuint64_t strides[2] = {(cuuint64_t)stride1 * 2, (cuuint64_t)stride2 * 2};
+    const cuuint32_t box[3] = {64, (cuuint32_t)box1, (cuuint32_t)box2};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_last_error("cuTensorMapEncodeTiled failed (base must be 16-byte aligned, strides multiples of 8 elements)");
+        return LLMB_ERR_INVALID;
+    }
+    return LLMB_OK;
+}
+
 }  // namespace llmb
 
 extern "C" int llmb_gemm_f16(const LlmbGemmArgs *a, llmb_stream_t stream_) {
