@@ -9,13 +9,24 @@
 //   the shortest prefix whose running sum reaches top_p is renormalised       (:1131-1148)
 //   the first entry whose running sum exceeds u is returned, entry 0 if none  (:1154-1160)
 //
-// One CTA of 1024 threads; thread t owns the vocabulary entries i = t (mod 1024).  The descending order is
-// never built for the whole vocabulary: entries are taken one at a time by a block-wide argmax (the owner of
-// the winner rescans its own entries), first top_k of them, then more only while the prefix has not reached
-// top_p (at most kSamplerMaxSelect in all).  The sequential part runs on thread 0 with the reference's
-// statements in the reference's order.  Different from the host code: the sum of the t_i is a tree over
-// threads, not a loop in index order, and expf is CUDA's, so probabilities can differ from the host's by a
-// few FP32 ulps; the token differs only if u lies within that distance of a boundary between two entries.
+// One cluster of 8 CTAs of 1024 threads (calls are one row each, so a row has to spread over several SMs itself).
+// Bound: latency of a chain of dependent passes; the data (256 KB for the 8B vocabulary) is 1/8 per CTA.
+//   t_i, sum   the vocabulary entries fall into 1024 classes i mod 1024; CTA c owns classes 128 c .. 128 c + 127 and keeps
+//              their t_i in shared memory (the caller's scratch for vocabularies beyond kSamplerSmemRows rows).  A class is
+//              added in index order by one thread, 32 classes by a warp butterfly, the 32 warps' sums by another: the
+//              sum does not depend on how many CTAs share the work.
+//   order      only the first `want` entries can matter: top_k of them, or kSamplerMaxSelect where top_p is so close to 1
+//              that rounding may carry the prefix past the first top_k (see want_entries).  A radix select over the 64-bit
+//              key (bits of p, then inverted index, so that keys are unique and equal p keep index order) finds a key
+//              prefix that between `want` and kSamplerCap entries reach: usually the first histogram (exponent and 3
+//              mantissa bits of p) does.  Those entries go to CTA 0, which sorts them.
+//   chain      the reference's statements on CTA 0: the running sums are one thread's, in the reference's order; the
+//              divisions between them are elementwise and use all threads.
+// Taking the entries one at a time by a block-wide argmax on a single CTA (every round: two barriers, and the owner's
+// rescan of its entries) took 495 us a draw at top_k 50 over 128256 entries; this form takes 20 us.
+// Different from the host code: the sum of the t_i is a tree over classes, not a loop in index order, and expf is CUDA's,
+// so probabilities can differ from the host's by a few FP32 ulps; the token differs only if u lies within that distance
+// of a boundary between two entries.
 #include "common.cuh"
 #include "../../include/llm_b200_synth.h"
 
@@ -23,6 +34,13 @@ namespace llmb {
 
 constexpr int kSamplerThreads = 1024;
 constexpr int kSamplerMaxSelect = 1024;
+constexpr int kSamplerCtas = 8;                                        // one portable cluster
+constexpr int kSamplerClasses = 1024;                                  // summation classes (index mod 1024)
+constexpr int kClassesPerCta = kSamplerClasses / kSamplerCtas;         // 128
+constexpr int kRowsPerPass = kSamplerThreads / kClassesPerCta;         // 8 rows of a CTA's classes at a time
+constexpr int kSamplerCap = 2048;                                      // entries that CTA 0 sorts at most
+constexpr int kSamplerSmemRows = 384;                                  // 192 KB of t_i per CTA: vocabularies up to 393216
+constexpr int kSamplerBins = 1024;
 
 struct SamplerParams {
     const __half *logits;
@@ -33,142 +51,226 @@ struct SamplerParams {
     int history_len;
     int *result;    // 0 ok, 1 overflow, 2 prefix longer than kSamplerMaxSelect
     int vocab, top_k;
+    int want;       // entries of the order that may be needed, top_k <= want <= kSamplerMaxSelect
+    int in_smem;    // t_i in shared memory (else in probs)
     float temperature, top_p, u;
 };
 
-__device__ __forceinline__ bool before(float pa, int ia, float pb, int ib) { return pa > pb || (pa == pb && ia < ib); }
+// Entries of the descending order that the chain can need.  The first k are renormalised to sum 1: their running sum
+// ends within 2 k 2^-24 < 1.3e-4 of 1 (k <= 1024 additions and as many divisions, each off by at most 2^-24), so the
+// prefix that reaches a top_p below 0.99 ends inside them.
+inline int want_entries(int vocab, int top_k, float top_p) {
+    if (top_p < 0.99f) return top_k;
+    return vocab < kSamplerMaxSelect ? vocab : kSamplerMaxSelect;
+}
+
+__device__ __forceinline__ uint32_t sampler_cta_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+__device__ __forceinline__ void sampler_cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+__device__ __forceinline__ uint32_t peer_smem(const void *own, uint32_t cta) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(own)), "r"(cta));
+    return r;
+}
+
+__device__ __forceinline__ uint64_t sample_key(float pr, int i) {
+    return ((uint64_t)__float_as_uint(pr) << 32) | (uint32_t)(0xffffffffu - (uint32_t)i);
+}
 
 __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerParams p) {
+    extern __shared__ float t_smem[];               // [rows][128] t_i, then p_i, of this CTA's classes
+    __shared__ float warp_sums[32];                 // of all CTAs
+    __shared__ int hist[kSamplerBins];
+    __shared__ int scan_s[32];
+    __shared__ int bin_s, above_s, count_s;         // threshold bin, entries above it, entries from it on
+    __shared__ int n_list;                          // CTA 0: entries collected
+    __shared__ uint64_t list[kSamplerCap];          // CTA 0
     __shared__ float sel_p[kSamplerMaxSelect];
-    __shared__ int sel_i[kSamplerMaxSelect];
-    __shared__ float red_v[32];
-    __shared__ int red_i[32];
-    __shared__ float total_s;
-    __shared__ int more_s;     // thread 0 wants one more entry of the order
-    __shared__ int winner_s;
+    __shared__ float sum_s;
+    __shared__ int cutoff_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t cta = sampler_cta_rank();
     pdl_launch_dependents();
     pdl_wait();
 
-    // ---- t_i and their sum ----
-    float local = 0.0f;
-    for (int i = tid; i < p.vocab; i += kSamplerThreads) {
-        const float t = expf(__fdiv_rn(__half2float(p.logits[i]), p.temperature));
-        p.probs[i] = t;
-        local += t;
+    // ---- t_i of this CTA's classes: thread = class cls, rows row0, row0 + 8, ... ----
+    const int cls = (int)cta * kClassesPerCta + (tid & (kClassesPerCta - 1)), row0 = tid / kClassesPerCta;
+    const int rows = (p.vocab + kSamplerClasses - 1) / kSamplerClasses;
+    // element (row, class) of the vocabulary: t[row * t_stride + (class within the CTA)]
+    float *t = p.in_smem ? t_smem : p.probs + (size_t)cta * kClassesPerCta;
+    const int t_stride = p.in_smem ? kClassesPerCta : kSamplerClasses, col = tid & (kClassesPerCta - 1);
+    for (int base = row0; base < rows; base += 8 * kRowsPerPass) {
+        __half x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {  // eight loads in flight
+            const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
+            x[j] = row < rows && i < p.vocab ? p.logits[i] : __half(0.0f);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
+            if (row < rows && i < p.vocab) t[(size_t)row * t_stride + col] = expf(__fdiv_rn(__half2float(x[j]), p.temperature));
+        }
     }
-    local = warp_sum(local);
-    if (lane == 0) red_v[warp] = local;
+    if (tid < kSamplerBins) hist[tid] = 0;
+    if (tid == 0) n_list = 0;
     __syncthreads();
-    if (warp == 0) {
-        float v = red_v[lane];
-        v = warp_sum(v);
-        if (lane == 0) total_s = v;
+    if (tid < kClassesPerCta) {  // here col == tid
+        float local = 0.0f;
+        const int n = cls < p.vocab ? (p.vocab - cls + kSamplerClasses - 1) / kSamplerClasses : 0;
+#pragma unroll 8
+        for (int row = 0; row < n; ++row) local += t[(size_t)row * t_stride + col];
+        local = warp_sum(local);
+        if (lane < kSamplerCtas)  // the same value in all lanes: lane c tells CTA c
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer_smem(&warp_sums[cta * (kClassesPerCta / 32) + warp], lane)), "f"(local) : "memory");
     }
-    __syncthreads();
-    const float total = total_s;
-    if (!(total > 0.0f) || isinf(total) || isnan(total)) {
-        if (tid == 0) { p.token_out[0] = -1; p.result[0] = 1; }
+    sampler_cluster_sync();
+    const float total = warp_sum(warp_sums[lane]);
+    if (!(total > 0.0f) || isinf(total) || isnan(total)) {  // the same in every thread of the cluster
+        if (cta == 0 && tid == 0) { p.token_out[0] = -1; p.result[0] = 1; }
         return;
     }
-    // ---- p_i; every thread's best entry ----
-    float best = -1.0f;
-    int best_i = 0x7fffffff;
-    for (int i = tid; i < p.vocab; i += kSamplerThreads) {
-        const float pr = __fdiv_rn(p.probs[i], total);
-        p.probs[i] = pr;
-        if (before(pr, i, best, best_i)) { best = pr; best_i = i; }
+
+    // ---- p_i, and a key prefix that enough entries reach ----
+    for (int row = row0; row < rows; row += kRowsPerPass) {
+        if (row * kSamplerClasses + cls >= p.vocab) break;
+        const float pr = __fdiv_rn(t[(size_t)row * t_stride + col], total);
+        t[(size_t)row * t_stride + col] = pr;
+        atomicAdd(&hist[__float_as_uint(pr) >> 20], 1);  // p <= 1: the bin is at most 0x3f8
     }
-    // ---- the order, one entry at a time ----
-    int n_sel = 0;
-    float sum_k = 0.0f, cumulative = 0.0f;  // thread 0's running values
-    int cutoff = -1;
+    uint64_t floor_key = 0;  // prefix of the keys that are taken, at `shift`
+    int shift = 52, need = p.want;
     for (;;) {
-        // block-wide argmax of the threads' best entries
-        float v = best;
-        int vi = best_i;
+        sampler_cluster_sync();  // the histograms of all CTAs are complete
+        int cnt = 0;
 #pragma unroll
-        for (int m = 16; m > 0; m >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, v, m);
-            const int oi = __shfl_xor_sync(0xffffffffu, vi, m);
-            if (before(ov, oi, v, vi)) { v = ov; vi = oi; }
+        for (int z = 0; z < kSamplerCtas; ++z) {
+            int v;
+            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(peer_smem(&hist[kSamplerBins - 1 - tid], z)) : "memory");
+            cnt += v;
         }
-        if (lane == 0) { red_v[warp] = v; red_i[warp] = vi; }
-        __syncthreads();
-        if (warp == 0) {
-            v = red_v[lane];
-            vi = red_i[lane];
+        // thread b holds bin 1023 - b: an inclusive scan counts the entries of that bin and all higher ones
+        int inc = cnt;
 #pragma unroll
-            for (int m = 16; m > 0; m >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, v, m);
-                const int oi = __shfl_xor_sync(0xffffffffu, vi, m);
-                if (before(ov, oi, v, vi)) { v = ov; vi = oi; }
-            }
-            if (lane == 0) {
-                sel_p[n_sel] = v;
-                sel_i[n_sel] = vi;
-                winner_s = vi;
-                // does the sequential part need another entry after this one?
-                int more = 1;
-                const int have = n_sel + 1;
-                if (have < p.top_k && have < p.vocab) {
-                    more = 1;                       // still collecting the first top_k entries
-                } else {
-                    if (have == p.top_k || (have == p.vocab && have < p.top_k)) {
-                        // top_k_sampling: renormalise the first k entries (inference.cu:1088-1096)
-                        for (int i = 0; i < have; ++i) sum_k += sel_p[i];
-                        for (int i = 0; i < have; ++i) sel_p[i] = __fdiv_rn(sel_p[i], sum_k);
-                        // top_p_sampling: running sum over the (partly renormalised) order (:1131-1136)
-                        for (int i = 0; i < have && cutoff < 0; ++i) {
-                            cumulative += sel_p[i];
-                            if (cumulative >= p.top_p) cutoff = i;
-                        }
-                    } else {  // an entry beyond the first k keeps its own probability
-                        cumulative += sel_p[have - 1];
-                        if (cumulative >= p.top_p) cutoff = have - 1;
-                    }
-                    more = (cutoff < 0 && have < p.vocab && have < kSamplerMaxSelect) ? 1 : 0;
-                }
-                more_s = more;
-            }
+        for (int m = 1; m < 32; m <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, inc, m);
+            if (lane >= m) inc += o;
+        }
+        if (lane == 31) scan_s[warp] = inc;
+        __syncthreads();
+        int before_warp = 0;
+        for (int w = 0; w < warp; ++w) before_warp += scan_s[w];
+        inc += before_warp;
+        if (inc >= need && inc - cnt < need) {
+            bin_s = kSamplerBins - 1 - tid;
+            above_s = inc - cnt;
+            count_s = inc;
         }
         __syncthreads();
-        ++n_sel;
-        if (!more_s) break;
-        // the owner of the winner strikes it out and finds its next best entry
-        const int w = winner_s;
-        if ((w % kSamplerThreads) == tid) {
-            p.probs[w] = -1.0f;
-            best = -1.0f;
-            best_i = 0x7fffffff;
-            for (int i = tid; i < p.vocab; i += kSamplerThreads) {
-                const float pr = p.probs[i];
-                if (pr >= 0.0f && before(pr, i, best, best_i)) { best = pr; best_i = i; }
-            }
+        floor_key += (uint64_t)bin_s;
+        // entries above the bins of this level were counted out of `need` already: they are among the taken ones too
+        if (p.want - need + count_s <= kSamplerCap || shift == 0) break;
+        need -= above_s;
+        const int bits = shift >= 10 ? 10 : shift;
+        const int next = shift - bits;
+        sampler_cluster_sync();  // every CTA has read the histograms
+        hist[tid] = 0;
+        __syncthreads();
+        for (int row = row0; row < rows; row += kRowsPerPass) {
+            const int i = row * kSamplerClasses + cls;
+            if (i >= p.vocab) break;
+            const uint64_t key = sample_key(t[(size_t)row * t_stride + col], i);
+            if ((key >> shift) == floor_key) atomicAdd(&hist[(int)(key >> next) & ((1 << bits) - 1)], 1);
+        }
+        floor_key <<= bits;
+        shift = next;
+    }
+    // ---- the entries that reach it go to CTA 0 ----
+    const uint32_t n_list0 = peer_smem(&n_list, 0), list0 = peer_smem(list, 0);
+    for (int row = row0; row < rows; row += kRowsPerPass) {
+        const int i = row * kSamplerClasses + cls;
+        if (i >= p.vocab) break;
+        const uint64_t key = sample_key(t[(size_t)row * t_stride + col], i);
+        if ((key >> shift) >= floor_key) {
+            int at;
+            asm volatile("atom.relaxed.cluster.shared::cluster.add.s32 %0, [%1], 1;" : "=r"(at) : "r"(n_list0) : "memory");
+            if (at < kSamplerCap) asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(list0 + (uint32_t)at * 8), "l"(key) : "memory");
         }
     }
+    sampler_cluster_sync();
+    if (cta != 0) return;
+
+    // ---- descending order of the collected keys (bitonic; the padding sorts last) ----
+    const int n = min(n_list, kSamplerCap);
+    int n2 = 32;
+    while (n2 < n) n2 <<= 1;
+    for (int i = n + tid; i < n2; i += kSamplerThreads) list[i] = 0;
+    __syncthreads();
+    for (int size = 2; size <= n2; size <<= 1)
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (tid < n2 / 2) {
+                const int a = 2 * tid - (tid & (stride - 1)), b = a + stride;
+                const uint64_t ka = list[a], kb = list[b];
+                if ((ka < kb) == ((a & size) == 0)) { list[a] = kb; list[b] = ka; }
+            }
+            __syncthreads();
+        }
+    const int have = min(p.want, n);  // n >= want: the threshold bin was chosen so
+    if (tid < have) sel_p[tid] = __uint_as_float((uint32_t)(list[tid] >> 32));
+    __syncthreads();
+    // ---- top_k_sampling: renormalise the first k entries (inference.cu:1088-1096) ----
+    const int k = min(p.top_k, have);
+    if (tid == 0) {
+        float sum_k = 0.0f;
+#pragma unroll 8
+        for (int i = 0; i < k; ++i) sum_k += sel_p[i];
+        sum_s = sum_k;
+    }
+    __syncthreads();
+    if (tid < k) sel_p[tid] = __fdiv_rn(sel_p[tid], sum_s);
+    __syncthreads();
+    // ---- top_p_sampling: the prefix whose running sum reaches top_p (:1131-1136); entries beyond the first k keep
+    // their own probability ----
+    if (tid == 0) {
+        float cumulative = 0.0f;
+        int cutoff = -1;
+        for (int i = 0; i < have; ++i) {
+            cumulative += sel_p[i];
+            if (cumulative >= p.top_p) { cutoff = i; break; }
+        }
+        if (cutoff < 0 && have == p.vocab) cutoff = p.vocab - 1;  // :1140-1143
+        cutoff_s = cutoff;
+        sum_s = cumulative;  // :1138
+    }
+    __syncthreads();
+    const int cutoff = cutoff_s;
+    if (cutoff < 0) {  // the prefix ran past what this kernel orders: let the host sampler take the step
+        if (tid == 0) { p.token_out[0] = -1; p.result[0] = 2; }
+        return;
+    }
+    if (tid <= cutoff) sel_p[tid] = __fdiv_rn(sel_p[tid], sum_s);  // :1146-1148
+    __syncthreads();
     if (tid != 0) return;
-    if (cutoff < 0) {
-        if (n_sel < p.vocab) {  // the prefix ran past what this kernel orders: let the host sampler take the step
-            p.token_out[0] = -1;
-            p.result[0] = 2;
-            return;
-        }
-        cutoff = p.vocab - 1;   // :1140-1143
-    }
-    const float sum = cumulative;  // :1138
-    for (int i = 0; i <= cutoff; ++i) sel_p[i] = __fdiv_rn(sel_p[i], sum);  // :1146-1148
-    int token = sel_i[0];          // :1159-1160
+    int at = 0;                    // :1159-1160
     float run = 0.0f;
     for (int i = 0; i <= cutoff; ++i) {  // :1154-1158
         run += sel_p[i];
-        if (p.u < run) { token = sel_i[i]; break; }
+        if (p.u < run) { at = i; break; }
     }
+    const int token = (int)(0xffffffffu - (uint32_t)list[at]);
     p.token_out[0] = token;
     p.result[0] = 0;
     if (p.pos && p.history) {
-        const int at = p.pos[0];
-        if (at >= 0 && at < p.history_len) p.history[at] = token;
+        const int where = p.pos[0];
+        if (where >= 0 && where < p.history_len) p.history[where] = token;
     }
 }
 
@@ -204,6 +306,13 @@ extern "C" int llmb_sample_logits(const uint16_t *d_logits, int vocab, float tem
     p.temperature = temperature;
     p.top_p = top_p;
     p.u = llmb_synth_uniform(llmb_stream_key(seed, LLMB_SID_SAMPLER), draw);
-    LLMB_CUDA_OK(launch_pdl(sample_kernel, dim3(1), dim3(kSamplerThreads), 0, static_cast<cudaStream_t>(stream_), use_pdl != 0, p));
+    p.want = want_entries(vocab, top_k, top_p);
+    const int rows = (vocab + kSamplerClasses - 1) / kSamplerClasses;
+    p.in_smem = rows <= kSamplerSmemRows ? 1 : 0;
+    const size_t smem = p.in_smem ? (size_t)rows * kClassesPerCta * sizeof(float) : 0;
+    static size_t attr_set[kMaxDevices] = {};
+    LLMB_CUDA_OK(ensure_dynamic_smem(sample_kernel, attr_set, smem));
+    LLMB_CUDA_OK(launch_pdl_cluster(sample_kernel, dim3(kSamplerCtas), dim3(kSamplerThreads), smem, static_cast<cudaStream_t>(stream_),
+                                    use_pdl != 0, dim3(kSamplerCtas, 1, 1), p));
     return LLMB_OK;
 }
