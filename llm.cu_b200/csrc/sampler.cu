@@ -23,7 +23,8 @@
 //   chain      the reference's statements on CTA 0: the running sums are one thread's, in the reference's order; the
 //              divisions between them are elementwise and use all threads.
 // Taking the entries one at a time by a block-wide argmax on a single CTA (every round: two barriers, and the owner's
-// rescan of its entries) took 495 us a draw at top_k 50 over 128256 entries; this form takes 20 us.
+// rescan of its entries) took 495 us a draw at top_k 50 over 128256 entries; this form takes 16 us (20 before short lists were ranked
+// by counting and the running sums lost their load and branch per entry).
 // Different from the host code: the sum of the t_i is a tree over classes, not a loop in index order, and expf is CUDA's,
 // so probabilities can differ from the host's by a few FP32 ulps; the token differs only if u lies within that distance
 // of a boundary between two entries.
@@ -41,6 +42,7 @@ constexpr int kRowsPerPass = kSamplerThreads / kClassesPerCta;         // 8 rows
 constexpr int kSamplerCap = 2048;                                      // entries that CTA 0 sorts at most
 constexpr int kSamplerSmemRows = 384;                                  // 192 KB of t_i per CTA: vocabularies up to 393216
 constexpr int kSamplerBins = 1024;
+constexpr int kRankThreads = 4, kSamplerRankCap = kSamplerThreads / kRankThreads;  // up to 256 keys are ranked by counting
 
 struct SamplerParams {
     const __half *logits;
@@ -83,6 +85,29 @@ __device__ __forceinline__ uint32_t peer_smem(const void *own, uint32_t cta) {
 
 __device__ __forceinline__ uint64_t sample_key(float pr, int i) {
     return ((uint64_t)__float_as_uint(pr) << 32) | (uint32_t)(0xffffffffu - (uint32_t)i);
+}
+
+// Index of the first entry whose running sum (in order, one rounding per entry) satisfies `hit`, -1 if none does; `run` =
+// the running sum up to it (or of all n).  No probability is negative, so a sum of eight is looked at only if its last
+// running value hits: the chain is then one addition per entry, not a load, an addition and a branch.
+template <typename Hit>
+__device__ __forceinline__ int first_reaching(const float *v, int n, float &run, const Hit &hit) {
+    int i = 0;
+    for (; i + 8 <= n; i += 8) {
+        float c[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) c[j] = v[i + j];
+        c[0] += run;
+#pragma unroll
+        for (int j = 1; j < 8; ++j) c[j] += c[j - 1];
+        if (hit(c[7])) break;
+        run = c[7];
+    }
+    for (; i < n; ++i) {
+        run += v[i];
+        if (hit(run)) return i;
+    }
+    return -1;
 }
 
 __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerParams p) {
@@ -166,9 +191,7 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
         }
         if (lane == 31) scan_s[warp] = inc;
         __syncthreads();
-        int before_warp = 0;
-        for (int w = 0; w < warp; ++w) before_warp += scan_s[w];
-        inc += before_warp;
+        inc += __reduce_add_sync(0xffffffffu, lane < warp ? scan_s[lane] : 0);
         if (inc >= need && inc - cnt < need) {
             bin_s = kSamplerBins - 1 - tid;
             above_s = inc - cnt;
@@ -208,21 +231,33 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     sampler_cluster_sync();
     if (cta != 0) return;
 
-    // ---- descending order of the collected keys (bitonic; the padding sorts last) ----
+    // ---- descending order of the collected keys ----
     const int n = min(n_list, kSamplerCap);
-    int n2 = 32;
-    while (n2 < n) n2 <<= 1;
-    for (int i = n + tid; i < n2; i += kSamplerThreads) list[i] = 0;
-    __syncthreads();
-    for (int size = 2; size <= n2; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            if (tid < n2 / 2) {
-                const int a = 2 * tid - (tid & (stride - 1)), b = a + stride;
-                const uint64_t ka = list[a], kb = list[b];
-                if ((ka < kb) == ((a & size) == 0)) { list[a] = kb; list[b] = ka; }
+    if (n <= kSamplerRankCap) {  // each key's rank by counting the greater ones, four threads per key: one barrier
+        const int i = tid / kRankThreads, part = tid % kRankThreads;
+        const uint64_t mine = i < n ? list[i] : 0;
+        int rank = 0;
+        for (int j = part; j < n; j += kRankThreads) rank += list[j] > mine ? 1 : 0;
+#pragma unroll
+        for (int m = 1; m < kRankThreads; m <<= 1) rank += __shfl_xor_sync(0xffffffffu, rank, m);
+        __syncthreads();
+        if (i < n && part == 0) list[rank] = mine;  // keys are unique: so are ranks
+        __syncthreads();
+    } else {
+        int n2 = 512;  // bitonic; the padding sorts last
+        while (n2 < n) n2 <<= 1;
+        for (int i = n + tid; i < n2; i += kSamplerThreads) list[i] = 0;
+        __syncthreads();
+        for (int size = 2; size <= n2; size <<= 1)
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                if (tid < n2 / 2) {
+                    const int a = 2 * tid - (tid & (stride - 1)), b = a + stride;
+                    const uint64_t ka = list[a], kb = list[b];
+                    if ((ka < kb) == ((a & size) == 0)) { list[a] = kb; list[b] = ka; }
+                }
+                __syncthreads();
             }
-            __syncthreads();
-        }
+    }
     const int have = min(p.want, n);  // n >= want: the threshold bin was chosen so
     if (tid < have) sel_p[tid] = __uint_as_float((uint32_t)(list[tid] >> 32));
     __syncthreads();
@@ -241,11 +276,7 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     // their own probability ----
     if (tid == 0) {
         float cumulative = 0.0f;
-        int cutoff = -1;
-        for (int i = 0; i < have; ++i) {
-            cumulative += sel_p[i];
-            if (cumulative >= p.top_p) { cutoff = i; break; }
-        }
+        int cutoff = first_reaching(sel_p, have, cumulative, [&](float run) { return run >= p.top_p; });
         if (cutoff < 0 && have == p.vocab) cutoff = p.vocab - 1;  // :1140-1143
         cutoff_s = cutoff;
         sum_s = cumulative;  // :1138
@@ -259,12 +290,9 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     if (tid <= cutoff) sel_p[tid] = __fdiv_rn(sel_p[tid], sum_s);  // :1146-1148
     __syncthreads();
     if (tid != 0) return;
-    int at = 0;                    // :1159-1160
-    float run = 0.0f;
-    for (int i = 0; i <= cutoff; ++i) {  // :1154-1158
-        run += sel_p[i];
-        if (p.u < run) { at = i; break; }
-    }
+    float run = 0.0f;  // :1154-1158
+    const int drawn = first_reaching(sel_p, cutoff + 1, run, [&](float r) { return p.u < r; });
+    const int at = drawn < 0 ? 0 : drawn;  // :1159-1160
     const int token = (int)(0xffffffffu - (uint32_t)list[at]);
     p.token_out[0] = token;
     p.result[0] = 0;
