@@ -198,9 +198,9 @@ int cache_debug_read(CudaCache *cache, int which, void *out, size_t bytes);
  * (consumers: entered, dependency met, input ready, done; finisher: started, first stage, last
  * stage, fenced). */
 int cache_debug_trace(CudaCache *cache, int enable);
-/* Prompt phase.  By default a run of >= 16 new prompt tokens goes through the block path: all but
- * the last token as blocks of up to 1024 rows (tensor-core projections, block attention), the last
- * one through the decode step for its logits.  enable = 0 feeds every prompt token through the
+/* Prompt phase.  By default a run of > 16 new prompt tokens goes through the block path: blocks of
+ * up to 4096 rows (tensor-core projections, block attention), the last row of which goes on to the
+ * logits.  enable = 0 feeds every prompt token through the
  * decode step instead; min_rows > 0 changes the threshold.  The block path needs the whole model
  * on this GPU (tp_size 1) and projection widths that are multiples of 128; otherwise the decode
  * step is used.  The reference runs its layer loop over all rows on every call
@@ -225,7 +225,8 @@ int cache_sample_next_token_device(CudaCache *cache, float temperature, int top_
  * KV cache of config.max_seq rows: K, V [n_layers][n_seqs][max_seq][n_kv].  Needs tp_size 1.
  *   cache_batch_init     allocates the batch state (n_seqs <= 128); the single-sequence state is untouched
  *   cache_batch_prefill  tokens [n_seqs][n_tokens]: all but the last token of every sequence go into its
- *                        cache as blocks of rows; the last one becomes the input of the next step
+ *                        cache as blocks of rows (short prompts share a block); the last one becomes the
+ *                        input of the next step
  *   cache_batch_step     one step; tokens (optional [n_seqs]) replaces the inputs (teacher forcing), else the
  *                        tokens sampled by the previous step are fed; h_logits (optional [n_seqs][vocab] FP16
  *                        bits) and next_tokens (optional [n_seqs]) receive the step's results

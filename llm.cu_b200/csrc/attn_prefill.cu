@@ -128,7 +128,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     };
     const int n_tiles0 = key_tiles(0), n_tiles1 = key_tiles(1), n_max = max(n_tiles0, n_tiles1);
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         prior_status = *reinterpret_cast<volatile int *>(p.status);
         mbar_init(&q_full, 1);
@@ -153,6 +152,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();                                     // this CTA has its tensor memory (see gemm_tc.cu)
     const uint32_t tmem_o = tmem + 2 * kPaKeys;                  // O tile t at + t * HD
     pdl_wait();                                                  // q and the new cache rows are the previous kernel's output
 

@@ -28,6 +28,7 @@ struct GemmParams {
     int n_q, n_kv, head_dim, pos0, max_pos;
     const int *row_pos;  // ROPE_KV, batched decode: cache position of each row; row r belongs to sequence r
     long long seq_stride;  // cache rows between consecutive sequences
+    int rows_per_seq;      // ROPE_KV without row_pos: row r = position pos0 + r % rows_per_seq of sequence r / rows_per_seq
     int stages;  // ring depth of this launch (<= kGemmMaxStages)
     // split-K: blockIdx.z takes a slice of K, partial accumulators meet in the workspace and the last
     // CTA of a tile to arrive adds them in slice order and runs the epilogue
@@ -128,12 +129,34 @@ int make_map(CUtensorMap *map, const void *base, int rows, int k, int box_rows);
 // the 128-byte swizzle; what lies outside reads as zero.
 int make_map_3d(CUtensorMap *map, const void *base, int d0, int d1, int d2, size_t stride1, size_t stride2, int box1, int box2);
 
-// The small-M path of llmb_gemm_f16 (gemm_smallm.cu): m <= 32 rows.
-int launch_gemm_smallm(const LlmbGemmArgs *a, cudaStream_t stream);
+// llmb_gemm_f16 for callers inside the library.  rows_per_seq > 0 (ROPE_KV without row_pos): the m rows are the
+// positions pos0 .. of m / rows_per_seq sequences, one after the other, whose caches are seq_stride rows apart.
+// pdl: programmatic stream serialization at any m (the weights must not be the previous kernel's output).
+int launch_gemm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream);
+
+// Its small-M path (gemm_smallm.cu): m <= 32 rows.
+int launch_gemm_smallm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream);
+
+// Position and cache row of row `row` of a ROPE_KV launch.
+__device__ __forceinline__ int kv_position(const GemmParams &p, int row, size_t &cache_row) {
+    if (p.row_pos) {
+        const int pos = __ldg(p.row_pos + row);
+        cache_row = (size_t)row * (size_t)p.seq_stride + (size_t)pos;
+        return pos;
+    }
+    const int seq = row / p.rows_per_seq, pos = p.pos0 + (row - seq * p.rows_per_seq);
+    cache_row = (size_t)seq * (size_t)p.seq_stride + (size_t)pos;
+    return pos;
+}
 
 // Causal attention of `len` new rows of each of n_seqs sequences (attn_prefill.cu); the caches of consecutive
 // sequences are seq_stride elements apart, q and out are [n_seqs * len][n_q_heads * head_dim].
 int launch_attn_prefill(const __half *q, const __half *k_cache, const __half *v_cache, int n_seqs, size_t seq_stride, int len, int pos0,
                         int n_q_heads, int n_kv_heads, int head_dim, __half *out, bool pdl, cudaStream_t stream);
+
+// llmb_embed_rope for a block of n_seqs * len rows: positions pos0 .. pos0 + len - 1 of each sequence, sequence s with its
+// ids (position 0 first) at tokens + s * token_stride (misc.cu).
+int launch_embed_rows(const __half *embed, const int *tokens, size_t token_stride, int n_seqs, int len, int pos0, int d_model,
+                      int vocab, int head_dim, float theta, __half *x, float *rope_cs, bool pdl, cudaStream_t stream);
 
 }  // namespace llmb

@@ -103,11 +103,11 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
     };
     if (threadIdx.x == 0) stamp(0);  // entry
-    // The next kernel may start its own weight stream as soon as an SM has room.  After a scattering projection
-    // the next kernel is the gather, which takes no wait of its own and reads the exchange counter and the
-    // residual rows at once: it is let go only after this kernel's wait, when every earlier kernel is complete.
+    // The next kernel may start its own weight stream as soon as an SM has room (and this CTA has its accumulator
+    // columns, see gemm_tc.cu).  After a scattering projection the next kernel is the gather, which takes no wait of its
+    // own and reads the exchange counter and the residual rows at once: it is let go only after this kernel's wait, when
+    // every earlier kernel is complete.
     const bool scatter = !DUAL && p.epilogue == LLMB_EPI_TP_SCATTER;
-    if (!scatter) pdl_launch_dependents();
     // a wait that gave up earlier (here or in another kernel) leaves the status word set: take no wait at all,
     // but still let the previous kernel finish first so that the order of the chain holds
     if (threadIdx.x == 0) prior_status = *reinterpret_cast<volatile int *>(p.status);
@@ -136,6 +136,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_slot;
+    if (!scatter) pdl_launch_dependents();
     if (threadIdx.x == 0) stamp(1);  // barriers and tensor memory ready
 
     if (warp == 0) {
@@ -286,11 +287,12 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             } else {  // LLMB_EPI_ROPE_KV: the pair (even n, n + 1) sits in neighbouring lanes
                 float2 cs[4];
                 int pos[4];
+                size_t cache_row[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int b = min(b0 + i, b_hi - 1);
                     cs[i] = is_v ? make_float2(1.0f, 0.0f) : __ldg(p.rope_cs + (size_t)b * half_dim + pair);
-                    pos[i] = p.row_pos ? __ldg(p.row_pos + b) : p.pos0 + b;
+                    pos[i] = kv_position(p, b, cache_row[i]);
                 }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -310,8 +312,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         if (is_q) {
                             p.c[(size_t)b * p.n_q + n] = out;
                         } else {
-                            const size_t cache_row = p.row_pos ? (size_t)b * (size_t)p.seq_stride + (size_t)pos[i] : (size_t)pos[i];
-                            if (pos[i] >= 0 && pos[i] < p.max_pos) (is_v ? p.v_cache : p.k_cache)[cache_row * p.n_kv + local] = out;
+                            if (pos[i] >= 0 && pos[i] < p.max_pos) (is_v ? p.v_cache : p.k_cache)[cache_row[i] * p.n_kv + local] = out;
                         }
                     }
                 }
@@ -328,7 +329,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
 }
 
-int launch_gemm_smallm(const LlmbGemmArgs *a, cudaStream_t stream) {
+int launch_gemm_smallm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream) {
     const bool dual = a->epilogue == LLMB_EPI_SWIGLU;
     CUtensorMap mw, mw2, mx;
     int rc;
@@ -346,6 +347,7 @@ int launch_gemm_smallm(const LlmbGemmArgs *a, cudaStream_t stream) {
     p.n_q = a->n_q; p.n_kv = a->n_kv; p.head_dim = a->head_dim; p.pos0 = a->pos0; p.max_pos = a->max_pos;
     p.row_pos = a->row_pos;
     p.seq_stride = a->seq_stride;
+    p.rows_per_seq = rows_per_seq > 0 ? rows_per_seq : a->m;
     p.trace = reinterpret_cast<unsigned long long *>(a->trace);
     p.tp_seq = nullptr;
     if (a->epilogue == LLMB_EPI_TP_SCATTER) {
@@ -376,11 +378,11 @@ int launch_gemm_smallm(const LlmbGemmArgs *a, cudaStream_t stream) {
     static size_t attr_set[2][kMaxDevices] = {};  // per instantiation and device
     if (dual) {
         LLMB_CUDA_OK(ensure_dynamic_smem(gemm_smallm_kernel<true>, attr_set[1], smem));
-        LLMB_CUDA_OK(launch_pdl_cluster(gemm_smallm_kernel<true>, dim3(tiles, p.splits), dim3(kGemmThreads), smem, stream, a->use_pdl != 0,
+        LLMB_CUDA_OK(launch_pdl_cluster(gemm_smallm_kernel<true>, dim3(tiles, p.splits), dim3(kGemmThreads), smem, stream, pdl,
                                         dim3(1, p.splits, 1), mw, mw2, mx, p));
     } else {
         LLMB_CUDA_OK(ensure_dynamic_smem(gemm_smallm_kernel<false>, attr_set[0], smem));
-        LLMB_CUDA_OK(launch_pdl_cluster(gemm_smallm_kernel<false>, dim3(tiles, p.splits), dim3(kGemmThreads), smem, stream, a->use_pdl != 0,
+        LLMB_CUDA_OK(launch_pdl_cluster(gemm_smallm_kernel<false>, dim3(tiles, p.splits), dim3(kGemmThreads), smem, stream, pdl,
                                         dim3(1, p.splits, 1), mw, mw2, mx, p));
     }
     return LLMB_OK;

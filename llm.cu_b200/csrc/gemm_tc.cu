@@ -60,7 +60,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // up more bounded waits behind it
     if (threadIdx.x == 0) prior_status = *reinterpret_cast<volatile int *>(p.status);
     __syncthreads();
-    if (prior_status != 0) return;
+    if (prior_status != 0) {
+        pdl_wait();
+        return;
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kGemmStages; ++s) {
             mbar_init(&full_bar[s], 1);
@@ -77,13 +80,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_slot;
+    // not before the accumulator columns are allocated: a CTA of the next kernel that took them first would wait for
+    // this one (griddepcontrol.wait) while this one waits for the columns
+    pdl_launch_dependents();
 
     if (warp == 0) {
         if (lane == 0) {
             bool ok = true;
-            for (int kt = kt_begin, i = 0; kt < kt_end && ok; ++kt, ++i) {
+            // the head of the weight stream does not depend on the previous kernel: ask for it first
+            const int head = min(kGemmStages, kt_end - kt_begin);
+            for (int i = 0; i < head; ++i) {
+                unsigned char *st = ring + (size_t)i * kStageBytes;
+                mbar_arrive_expect_tx(&full_bar[i], kStageBytes);
+                tma_load_2d(st + kATileBytes, &map_b, (kt_begin + i) * kBK, n0, &full_bar[i]);
+                if (DUAL) tma_load_2d(st + kATileBytes + kBTileBytes, &map_b2, (kt_begin + i) * kBK, n0, &full_bar[i]);
+            }
+            pdl_wait();  // the activations are the previous kernel's output
+            for (int i = 0; i < head; ++i) tma_load_2d(ring + (size_t)i * kStageBytes, &map_a, (kt_begin + i) * kBK, m0, &full_bar[i]);
+            for (int kt = kt_begin + head, i = head; kt < kt_end && ok; ++kt, ++i) {
                 const int s = i % kGemmStages;
-                if (i >= kGemmStages) ok = mbar_wait(&empty_bar[s], ((i / kGemmStages) - 1) & 1, p.status, 301);
+                ok = mbar_wait(&empty_bar[s], ((i / kGemmStages) - 1) & 1, p.status, 301);
                 if (!ok) break;
                 unsigned char *st = ring + (size_t)s * kStageBytes;
                 mbar_arrive_expect_tx(&full_bar[s], kStageBytes);
@@ -118,6 +134,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // ---- epilogue: thread = one row of the tile, TMEM lanes (warp % 4) * 32 .. + 32 ----
         const bool ok = mbar_wait(&acc_bar, 0, p.status, 303);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        pdl_wait();  // from here on global memory of earlier kernels is read and written
         const int lane_group = (warp & 3) * 32;
         const int row = m0 + lane_group + lane;
         const bool row_ok = ok && row < p.M;
@@ -216,8 +233,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                 for (int i = 0; i < 4; ++i) dst[i] = reinterpret_cast<const uint4 *>(out)[i];
             } else {  // LLMB_EPI_ROPE_KV
-                const int pos = p.row_pos ? __ldg(p.row_pos + row) : p.pos0 + row;
-                const size_t cache_row = p.row_pos ? (size_t)row * (size_t)p.seq_stride + (size_t)pos : (size_t)pos;
+                size_t cache_row;
+                const int pos = kv_position(p, row, cache_row);
                 const int half_dim = p.head_dim >> 1;
                 const bool is_v = col0 >= p.n_q + p.n_kv;
 #pragma unroll
@@ -314,7 +331,10 @@ int make_map_3d(CUtensorMap *map, const void *base, int d0, int d1, int d2, size
 }  // namespace llmb
 
 extern "C" int llmb_gemm_f16(const LlmbGemmArgs *a, llmb_stream_t stream_) {
-    using namespace llmb;
+    return llmb::launch_gemm(a, 0, a && a->use_pdl != 0 && a->m <= 32 && a->tile_n == 0, static_cast<cudaStream_t>(stream_));
+}
+
+int llmb::launch_gemm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream) {
     if (!a || !a->a || !a->b || (!a->c && a->epilogue != LLMB_EPI_TP_SCATTER) || a->m <= 0 || a->n <= 0 || a->k <= 0) return LLMB_ERR_INVALID;
     const bool small_m = a->m <= 32 && a->tile_n == 0;
     // the weight-streaming kernel masks the tail of its last tile, so STORE / TP_SCATTER take any n there
@@ -337,7 +357,7 @@ extern "C" int llmb_gemm_f16(const LlmbGemmArgs *a, llmb_stream_t stream_) {
         return LLMB_ERR_INVALID;
     }
     // A handful of rows (batched decode): the weight-streaming kernel with the operands swapped
-    if (small_m) return launch_gemm_smallm(a, static_cast<cudaStream_t>(stream_));
+    if (small_m) return launch_gemm_smallm(a, rows_per_seq, pdl, stream);
     // Small grids: with a workspace, 128-wide tiles and K split across CTAs until the SMs are covered
     // (every CTA then streams its own weights and only its slice of the activations); without one, the
     // widest tile that still gives every SM a CTA.
@@ -370,6 +390,7 @@ extern "C" int llmb_gemm_f16(const LlmbGemmArgs *a, llmb_stream_t stream_) {
     p.n_q = a->n_q; p.n_kv = a->n_kv; p.head_dim = a->head_dim; p.pos0 = a->pos0; p.max_pos = a->max_pos;
     p.row_pos = a->row_pos;
     p.seq_stride = a->seq_stride;
+    p.rows_per_seq = rows_per_seq > 0 ? rows_per_seq : a->m;
     dim3 grid(m_tiles, a->n / bn);
     const int tiles = (int)(grid.x * grid.y), k_tiles = a->k / kBK;
     p.splits = 1;
@@ -389,13 +410,11 @@ extern "C" int llmb_gemm_f16(const LlmbGemmArgs *a, llmb_stream_t stream_) {
         if (p.stages > kGemmMaxStages) p.stages = kGemmMaxStages;
     }
     const size_t smem = (size_t)p.stages * gemm_stage_bytes(dual, bn) + 1024;
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     void (*kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const GemmParams) =
         dual ? (bn == 128 ? gemm_tc_kernel<true, 128> : bn == 64 ? gemm_tc_kernel<true, 64> : gemm_tc_kernel<true, 32>)
              : (bn == 128 ? gemm_tc_kernel<false, 128> : bn == 64 ? gemm_tc_kernel<false, 64> : gemm_tc_kernel<false, 32>);
     static size_t attr_set[2][3][kMaxDevices] = {};  // per instantiation and device
     LLMB_CUDA_OK(ensure_dynamic_smem(kernel, attr_set[dual ? 1 : 0][bn == 128 ? 0 : bn == 64 ? 1 : 2], smem));
-    kernel<<<grid, kGemmThreads, smem, stream>>>(ma, mb, mb2, p);
-    LLMB_CUDA_OK(cudaGetLastError());
+    LLMB_CUDA_OK(launch_pdl(kernel, grid, dim3(kGemmThreads), smem, stream, pdl, ma, mb, mb2, p));
     return LLMB_OK;
 }

@@ -1,6 +1,6 @@
 // Small kernels around the projections: load-time BF16->FP16 conversion, synthetic weights,
 // the step prologue (embedding row + RoPE angles) and the greedy-argmax step epilogue.
-#include "common.cuh"
+#include "gemm_common.cuh"
 
 #include "../../include/llm_b200_synth.h"
 
@@ -74,17 +74,21 @@ __global__ void fill_u16_kernel(uint16_t *out, uint16_t value, uint64_t n) {
 // ---------------------------------------------------------------------------------------
 __global__ void embed_rope_kernel(const __half *__restrict__ embed, const int *__restrict__ tokens,
                                   const int *__restrict__ pos, int d_model, int vocab, int head_dim, float theta,
-                                  __half *__restrict__ x, float2 *__restrict__ rope_cs, int tokens_by_pos) {
+                                  __half *__restrict__ x, float2 *__restrict__ rope_cs, int tokens_by_pos, int pos0, int rows_per_seq,
+                                  size_t token_stride) {
     pdl_launch_dependents();
     pdl_wait();
     const int row = blockIdx.x;
-    int tok = tokens[tokens_by_pos ? pos[row] : row];
+    // rows_per_seq > 0: a block of several sequences, row = position pos0 + i of sequence s, whose ids start at s * token_stride
+    const int seq = rows_per_seq > 0 ? row / rows_per_seq : 0;
+    const int at = rows_per_seq > 0 ? pos0 + (row - seq * rows_per_seq) : pos[row];
+    int tok = tokens[rows_per_seq > 0 ? (size_t)seq * token_stride + (size_t)at : (size_t)(tokens_by_pos ? at : row)];
     tok = tok < 0 ? 0 : (tok >= vocab ? vocab - 1 : tok);
     const uint4 *src = reinterpret_cast<const uint4 *>(embed + (size_t)tok * d_model);
     uint4 *dst = reinterpret_cast<uint4 *>(x + (size_t)row * d_model);
     for (int i = threadIdx.x; i < d_model / 8; i += blockDim.x) dst[i] = __ldg(src + i);
     const int half_dim = head_dim / 2;
-    const float fpos = (float)pos[row];
+    const float fpos = (float)at;
     for (int i = threadIdx.x; i < half_dim; i += blockDim.x) {
         float freq = 1.0f / powf(theta, 2.0f * (float)i / (float)head_dim);
         float angle = fpos * freq;
@@ -250,7 +254,14 @@ extern "C" int llmb_embed_rope(const uint16_t *d_embed, const int32_t *d_tokens,
     LLMB_CUDA_OK(launch_pdl(embed_rope_kernel, dim3(n_rows), dim3(256), 0, static_cast<cudaStream_t>(stream_), use_pdl != 0,
                             reinterpret_cast<const __half *>(d_embed), d_tokens, d_pos, d_model, vocab, head_dim,
                             rope_theta, reinterpret_cast<__half *>(d_x), reinterpret_cast<float2 *>(d_rope_cs),
-                            tokens_by_pos));
+                            tokens_by_pos, 0, 0, 0));
+    return LLMB_OK;
+}
+
+int llmb::launch_embed_rows(const __half *embed, const int *tokens, size_t token_stride, int n_seqs, int len, int pos0, int d_model,
+                            int vocab, int head_dim, float theta, __half *x, float *rope_cs, bool pdl, cudaStream_t stream) {
+    LLMB_CUDA_OK(launch_pdl(embed_rope_kernel, dim3(n_seqs * len), dim3(256), 0, stream, pdl, embed, tokens, static_cast<const int *>(nullptr),
+                            d_model, vocab, head_dim, theta, x, reinterpret_cast<float2 *>(rope_cs), 0, pos0, len, token_stride));
     return LLMB_OK;
 }
 

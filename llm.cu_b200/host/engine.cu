@@ -28,7 +28,7 @@
 #include <map>
 #include <vector>
 
-#include "../csrc/common.cuh"
+#include "../csrc/gemm_common.cuh"
 #include "../../include/llama3.h"
 #include "host_internal.h"
 
@@ -80,7 +80,7 @@ struct Engine {
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     // prompt phase: blocks of rows through the tensor-core projections
     bool batched_prefill = true;
-    int prefill_min_rows = 16, prefill_chunk = 1024, pf_rows = 0;
+    int prefill_min_rows = 16, prefill_chunk = 4096, pf_rows = 0;
     __half *pf_x = nullptr, *pf_xn = nullptr, *pf_q = nullptr, *pf_attn = nullptr, *pf_h = nullptr;
     float *pf_rope = nullptr;
     int *pf_pos = nullptr;
@@ -355,78 +355,101 @@ int ensure_prefill_buffers(Engine *e, int rows) {
     return LLMB_OK;
 }
 
-// Appends the K/V rows of history positions [from, to) to the cache, a block of rows at a time:
-// the reference's layer loop (inference.cu:157-186) with every projection a tensor-core GEMM over
-// the block.  No logits: the caller runs the last prompt token through the decode step.
-// `ids` = the sequence's token ids on the device (position 0 first); kbase/vbase = layer 0 of the sequence's
-// cache; layer_stride = elements between consecutive layers of that cache.
-int prefill_rows(Engine *e, int from, int to, const int *ids, __half *kbase, __half *vbase, size_t layer_stride) {
+// One block of the prompt phase: positions pos0 .. pos0 + len - 1 of n_seqs sequences go through the reference's layer
+// loop (inference.cu:157-186) with every projection a tensor-core GEMM over all n_seqs * len rows.  `ids` = token ids on
+// the device (position 0 first), id_stride apart per sequence; kbase / vbase = layer 0 of the first sequence's cache,
+// whose layers are layer_stride elements apart and whose sequences max_seq rows.  What a block leaves behind is its K/V
+// rows, so the last layer ends with them, except for the very last row of a prompt whose logits are wanted (want_last;
+// n_seqs = 1): that row alone goes through the rest of the last layer and is left in pf_x at its place.
+int prefill_block(Engine *e, const int *ids, size_t id_stride, int n_seqs, int len, int pos0, __half *kbase, __half *vbase,
+                  size_t layer_stride, bool want_last) {
     Llama3 *m = e->model;
     const Llama3Config &c = m->config;
     cudaStream_t s = e->stream;
-    const int n_q = e->nq * e->hd, n_kv = e->nkv * e->hd;
-    int rc = ensure_prefill_buffers(e, std::min(to - from, e->prefill_chunk));
-    if (rc) return rc;
+    const int n_q = e->nq * e->hd, n_kv = e->nkv * e->hd, rows = n_seqs * len;
     auto u16 = [](const void *p) { return reinterpret_cast<const uint16_t *>(p); };
     auto u16w = [](void *p) { return reinterpret_cast<uint16_t *>(p); };
-    for (int p0 = from; p0 < to; p0 += e->prefill_chunk) {
-        const int rows = std::min(e->prefill_chunk, to - p0);
-        if ((rc = llmb_iota_i32(e->pf_pos, p0, rows, s))) return rc;
-        if ((rc = llmb_embed_rope(u16(m->embed_tokens->d_fp16_tensor), ids + p0, e->pf_pos, rows, e->d,
-                                  e->embed_rows, e->hd, c.rope_theta, u16w(e->pf_x), e->pf_rope, 0, 0, s)))
+    auto gemm = [&](const __half *a, const void *b, __half *out, int rows_, int n, int k, int epilogue) {
+        LlmbGemmArgs g = {};
+        g.a = u16(a); g.b = u16(b); g.c = u16w(out);
+        g.m = rows_; g.n = n; g.k = k;
+        g.epilogue = epilogue;
+        g.workspace = e->pf_ws; g.workspace_bytes = e->pf_ws_bytes;
+        return g;
+    };
+    int rc;
+    // the first kernel of a block takes no programmatic launch: the ids before it are a copy's output
+    if ((rc = launch_embed_rows(reinterpret_cast<const __half *>(m->embed_tokens->d_fp16_tensor), ids, id_stride, n_seqs, len, pos0, e->d,
+                                e->embed_rows, e->hd, c.rope_theta, e->pf_x, e->pf_rope, false, s)))
+        return rc;
+    e->launches += 1;
+    for (int l = 0; l < e->layers; ++l) {
+        const Llama3Layer *L = m->layers[l];
+        __half *kl = kbase + (size_t)l * layer_stride;
+        __half *vl = vbase + (size_t)l * layer_stride;
+        if ((rc = llmb_rmsnorm_rows(u16(e->pf_x), u16(L->input_layernorm->d_fp16_tensor), u16w(e->pf_xn), rows, e->d, c.eps, s)))
             return rc;
-        for (int l = 0; l < e->layers; ++l) {
-            const Llama3Layer *L = m->layers[l];
-            __half *kl = kbase + (size_t)l * layer_stride;
-            __half *vl = vbase + (size_t)l * layer_stride;
-            if ((rc = llmb_rmsnorm_rows(u16(e->pf_x), u16(L->input_layernorm->d_fp16_tensor), u16w(e->pf_xn), rows, e->d,
-                                        c.eps, s)))
-                return rc;
-            LlmbGemmArgs g = {};
-            g.a = u16(e->pf_xn);
-            g.b = u16(L->self_attn_q_proj->d_fp16_tensor);  // q, k, v rows are one contiguous buffer
-            g.c = u16w(e->pf_q);
-            g.m = rows; g.n = n_q + 2 * n_kv; g.k = e->d;
-            g.epilogue = LLMB_EPI_ROPE_KV;
-            g.n_q = n_q; g.n_kv = n_kv; g.head_dim = e->hd;
-            g.rope_cs = e->pf_rope;
-            g.k_cache = u16w(kl); g.v_cache = u16w(vl);
-            g.pos0 = p0; g.max_pos = e->max_seq;
-            g.workspace = e->pf_ws; g.workspace_bytes = e->pf_ws_bytes;
-            if ((rc = llmb_gemm_f16(&g, s))) return rc;
-            if ((rc = llmb_attn_prefill(u16(e->pf_q), u16(kl), u16(vl), rows, p0, e->nq, e->nkv, e->hd, u16w(e->pf_attn), s)))
-                return rc;
-            LlmbGemmArgs o = {};
-            o.a = u16(e->pf_attn);
-            o.b = u16(L->self_attn_o_proj->d_fp16_tensor);
-            o.c = u16w(e->pf_x);
-            o.m = rows; o.n = e->d; o.k = n_q;
-            o.epilogue = LLMB_EPI_RESIDUAL;
-            o.workspace = e->pf_ws; o.workspace_bytes = e->pf_ws_bytes;
-            if ((rc = llmb_gemm_f16(&o, s))) return rc;
-            if ((rc = llmb_rmsnorm_rows(u16(e->pf_x), u16(L->post_attention_layernorm->d_fp16_tensor), u16w(e->pf_xn), rows,
-                                        e->d, c.eps, s)))
-                return rc;
-            LlmbGemmArgs f = {};
-            f.a = u16(e->pf_xn);
-            f.b = u16(L->mlp_gate_proj->d_fp16_tensor);
-            f.b2 = u16(L->mlp_up_proj->d_fp16_tensor);
-            f.c = u16w(e->pf_h);
-            f.m = rows; f.n = e->ffn; f.k = e->d;
-            f.epilogue = LLMB_EPI_SWIGLU;
-            f.workspace = e->pf_ws; f.workspace_bytes = e->pf_ws_bytes;
-            if ((rc = llmb_gemm_f16(&f, s))) return rc;
-            LlmbGemmArgs dn = {};
-            dn.a = u16(e->pf_h);
-            dn.b = u16(L->mlp_down_proj->d_fp16_tensor);
-            dn.c = u16w(e->pf_x);
-            dn.m = rows; dn.n = e->d; dn.k = e->ffn;
-            dn.epilogue = LLMB_EPI_RESIDUAL;
-            dn.workspace = e->pf_ws; dn.workspace_bytes = e->pf_ws_bytes;
-            if ((rc = llmb_gemm_f16(&dn, s))) return rc;
+        LlmbGemmArgs g = gemm(e->pf_xn, L->self_attn_q_proj->d_fp16_tensor /* q, k, v rows are one contiguous buffer */, e->pf_q, rows,
+                              n_q + 2 * n_kv, e->d, LLMB_EPI_ROPE_KV);
+        g.n_q = n_q; g.n_kv = n_kv; g.head_dim = e->hd;
+        g.rope_cs = e->pf_rope;
+        g.k_cache = u16w(kl); g.v_cache = u16w(vl);
+        g.pos0 = pos0; g.max_pos = e->max_seq; g.seq_stride = e->max_seq;
+        if ((rc = launch_gemm(&g, len, true, s))) return rc;
+        e->launches += 2;
+        int first = 0, left = rows;  // rows that go on
+        if (l + 1 == e->layers) {
+            if (!want_last) break;
+            first = rows - 1;
+            left = 1;
         }
-        e->launches += 2 + 7 * e->layers;
+        __half *x = e->pf_x + (size_t)first * e->d;
+        if ((rc = launch_attn_prefill(e->pf_q + (size_t)first * n_q, kl, vl, n_seqs, (size_t)e->max_seq * n_kv, left / n_seqs, pos0 + first,
+                                      e->nq, e->nkv, e->hd, e->pf_attn, true, s)))
+            return rc;
+        g = gemm(e->pf_attn, L->self_attn_o_proj->d_fp16_tensor, x, left, e->d, n_q, LLMB_EPI_RESIDUAL);
+        if ((rc = launch_gemm(&g, 0, true, s))) return rc;
+        if ((rc = llmb_rmsnorm_rows(u16(x), u16(L->post_attention_layernorm->d_fp16_tensor), u16w(e->pf_xn), left, e->d, c.eps, s)))
+            return rc;
+        g = gemm(e->pf_xn, L->mlp_gate_proj->d_fp16_tensor, e->pf_h, left, e->ffn, e->d, LLMB_EPI_SWIGLU);
+        g.b2 = u16(L->mlp_up_proj->d_fp16_tensor);
+        if ((rc = launch_gemm(&g, 0, true, s))) return rc;
+        g = gemm(e->pf_h, L->mlp_down_proj->d_fp16_tensor, x, left, e->d, e->ffn, LLMB_EPI_RESIDUAL);
+        if ((rc = launch_gemm(&g, 0, true, s))) return rc;
+        e->launches += 5;
     }
+    return LLMB_OK;
+}
+
+// History positions [from, to) of one sequence, a block of up to prefill_chunk rows at a time; the K/V rows go to the
+// cache.  logits: the last row goes on to the logits and the greedy token, as a decode step would leave them (*d_pos
+// and the history advance).  `ids`, kbase, vbase, layer_stride as in prefill_block.
+int prefill_rows(Engine *e, int from, int to, const int *ids, __half *kbase, __half *vbase, size_t layer_stride, bool logits) {
+    int rc = ensure_prefill_buffers(e, std::min(to - from, e->prefill_chunk));
+    if (rc) return rc;
+    int last = 0;
+    for (int p0 = from; p0 < to; p0 += e->prefill_chunk) {
+        last = std::min(e->prefill_chunk, to - p0);
+        if ((rc = prefill_block(e, ids, 0, 1, last, p0, kbase, vbase, layer_stride, logits && p0 + last == to))) return rc;
+    }
+    if (!logits) return LLMB_OK;
+    if ((rc = set_device_int(e, e->d_pos, to - 1))) return rc;
+    LlmbGemvArgs lm = {};
+    lm.use_pdl = e->use_pdl ? 1 : 0;
+    lm.w = reinterpret_cast<const uint16_t *>(e->model->lm_head->d_fp16_tensor);
+    lm.x = reinterpret_cast<const uint16_t *>(e->pf_x + (size_t)(last - 1) * e->d);
+    lm.y = reinterpret_cast<uint16_t *>(e->logits);
+    lm.n = e->vocab;
+    lm.k = e->d;
+    lm.prologue = LLMB_PRO_RMSNORM;
+    lm.gamma = reinterpret_cast<const uint16_t *>(e->model->norm->d_fp16_tensor);
+    lm.eps = e->model->config.eps;
+    lm.epilogue = LLMB_EPI_STORE;
+    if ((rc = llmb_gemv_f16(&lm, e->stream))) return rc;
+    if ((rc = llmb_argmax_f16(reinterpret_cast<const uint16_t *>(e->logits), e->vocab, e->d_next, e->d_pos, e->d_history, e->max_seq + 1,
+                              lm.use_pdl, e->stream)))
+        return rc;
+    e->launches += 2;
     return LLMB_OK;
 }
 
@@ -533,9 +556,13 @@ int feed_tokens(Engine *e, const int *ids, int from, int to) {
     LLMB_CUDA_OK(cudaMemcpyAsync(e->d_history + from, ids + from, sizeof(int) * (size_t)(to - from),
                                  cudaMemcpyHostToDevice, e->stream));
     int rc, first = from;
-    // all but the last token as blocks of rows; the last one through the decode step, for its logits
     if (e->batched_prefill && to - 1 - from >= e->prefill_min_rows && prefill_supported(e)) {
-        if ((rc = prefill_rows(e, from, to - 1, e->d_history, e->kcache, e->vcache, (size_t)e->max_seq * e->nkv * e->hd))) return rc;
+        // one pass over the weights gives the cache rows and the last token's logits.  The projection of a single row onto
+        // the vocabulary takes d_model up to 8192 (llmb_gemv_f16); beyond, the last token is a decode step
+        const bool logits = e->d <= 8192;
+        if ((rc = prefill_rows(e, from, logits ? to : to - 1, e->d_history, e->kcache, e->vcache, (size_t)e->max_seq * e->nkv * e->hd, logits)))
+            return rc;
+        if (logits) return LLMB_OK;
         first = to - 1;
     } else if (e->batched_prefill && to - 1 - from >= e->prefill_min_rows && tp_rows_supported(e)) {
         if ((rc = prefill_rows_tp(e, from, to - 1, e->d_history, e->kcache, e->vcache, (size_t)e->max_seq * e->nkv * e->hd))) return rc;
@@ -1245,21 +1272,25 @@ extern "C" int cache_batch_prefill(CudaCache *cache, const int *tokens, int n_to
         return LLMB_ERR_INVALID;
     }
     const int B = e->bt_seqs;
-    const size_t n_kv = (size_t)e->nkv * e->hd;
+    const size_t n_kv = (size_t)e->nkv * e->hd, layer_stride = (size_t)B * e->max_seq * n_kv, id_stride = (size_t)e->max_seq + 1;
     std::vector<int> last((size_t)B), pos((size_t)B, n_tokens - 1);
     int rc;
-    for (int b = 0; b < B; ++b) {
-        int *hist = e->bt_history + (size_t)b * (e->max_seq + 1);
-        LLMB_CUDA_OK(cudaMemcpyAsync(hist, tokens + (size_t)b * n_tokens, sizeof(int) * (size_t)n_tokens, cudaMemcpyHostToDevice,
-                                     e->stream));
-        if (n_tokens > 1) {
-            __half *kb = e->bt_kcache + (size_t)b * e->max_seq * n_kv, *vb = e->bt_vcache + (size_t)b * e->max_seq * n_kv;
-            rc = e->tp_size > 1 ? prefill_rows_tp(e, 0, n_tokens - 1, hist, kb, vb, (size_t)B * e->max_seq * n_kv)
-                                : prefill_rows(e, 0, n_tokens - 1, hist, kb, vb, (size_t)B * e->max_seq * n_kv);
-            if (rc) return rc;
-        }
-        last[(size_t)b] = tokens[(size_t)b * n_tokens + n_tokens - 1];
+    LLMB_CUDA_OK(cudaMemcpy2DAsync(e->bt_history, sizeof(int) * id_stride, tokens, sizeof(int) * (size_t)n_tokens,
+                                   sizeof(int) * (size_t)n_tokens, (size_t)B, cudaMemcpyHostToDevice, e->stream));
+    // short prompts share blocks: as many whole sequences as fit one, so that the weights are read once for all of them
+    const int len = n_tokens - 1;
+    const int group = e->tp_size > 1 || len < 1 ? 1 : std::max(1, std::min(B, e->prefill_chunk / len));
+    if (e->tp_size == 1 && len > 0 && (rc = ensure_prefill_buffers(e, std::min(group * len, e->prefill_chunk)))) return rc;
+    for (int b = 0; b < B && len > 0; b += group) {
+        const int n = std::min(group, B - b);
+        const int *hist = e->bt_history + (size_t)b * id_stride;
+        __half *kb = e->bt_kcache + (size_t)b * e->max_seq * n_kv, *vb = e->bt_vcache + (size_t)b * e->max_seq * n_kv;
+        if (e->tp_size > 1) rc = prefill_rows_tp(e, 0, len, hist, kb, vb, layer_stride);
+        else if (group > 1) rc = prefill_block(e, hist, id_stride, n, len, 0, kb, vb, layer_stride, false);
+        else rc = prefill_rows(e, 0, len, hist, kb, vb, layer_stride, false);
+        if (rc) return rc;
     }
+    for (int b = 0; b < B; ++b) last[(size_t)b] = tokens[(size_t)b * n_tokens + n_tokens - 1];
     LLMB_CUDA_OK(cudaMemcpyAsync(e->bt_tok, last.data(), sizeof(int) * (size_t)B, cudaMemcpyHostToDevice, e->stream));
     LLMB_CUDA_OK(cudaMemcpyAsync(e->bt_pos, pos.data(), sizeof(int) * (size_t)B, cudaMemcpyHostToDevice, e->stream));
     if ((rc = queue_status_read(e))) return rc;
