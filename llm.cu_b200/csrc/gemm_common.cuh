@@ -122,6 +122,76 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 __device__ __forceinline__ float silu_gemm(float x) { return __fdiv_rn(x, 1.0f + expf(-x)); }
 
 
+// Position and cache row of row `row` of a ROPE_KV launch.
+__device__ __forceinline__ int kv_position(const GemmParams &p, int row, size_t &cache_row) {
+    if (p.row_pos) {
+        const int pos = __ldg(p.row_pos + row);
+        cache_row = (size_t)row * (size_t)p.seq_stride + (size_t)pos;
+        return pos;
+    }
+    const int seq = row / p.rows_per_seq, pos = p.pos0 + (row - seq * p.rows_per_seq);
+    cache_row = (size_t)seq * (size_t)p.seq_stride + (size_t)pos;
+    return pos;
+}
+
+// Epilogue of 32 accumulator columns (col0 .. col0 + 31, a multiple of 32) of one output row; u = the second
+// accumulator (up) of a SwiGLU projection.
+template <bool DUAL>
+__device__ __forceinline__ void finish_cols(const GemmParams &p, int row, int col0, const uint32_t (&v)[32], const uint32_t (&u)[32]) {
+    __align__(16) __half out[32];
+    if (DUAL) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) out[i] = __float2half_rn(silu_gemm(__uint_as_float(v[i])) * __uint_as_float(u[i]));
+        uint4 *dst = reinterpret_cast<uint4 *>(p.c + (size_t)row * p.N + col0);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dst[i] = reinterpret_cast<const uint4 *>(out)[i];
+    } else if (p.epilogue == LLMB_EPI_STORE) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) out[i] = __float2half_rn(__uint_as_float(v[i]));
+        uint4 *dst = reinterpret_cast<uint4 *>(p.c + (size_t)row * p.N + col0);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dst[i] = reinterpret_cast<const uint4 *>(out)[i];
+    } else if (p.epilogue == LLMB_EPI_RESIDUAL) {
+        uint4 *dst = reinterpret_cast<uint4 *>(p.c + (size_t)row * p.N + col0);
+        __align__(16) __half res[32];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) reinterpret_cast<uint4 *>(res)[i] = dst[i];
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            out[i] = __float2half_rn(__half2float(__float2half_rn(__uint_as_float(v[i]))) + __half2float(res[i]));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dst[i] = reinterpret_cast<const uint4 *>(out)[i];
+    } else {  // LLMB_EPI_ROPE_KV
+        size_t cache_row;
+        const int pos = kv_position(p, row, cache_row);
+        const int half_dim = p.head_dim >> 1;
+        const bool is_v = col0 >= p.n_q + p.n_kv;
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+            const float e = __half2float(__float2half_rn(__uint_as_float(v[i])));
+            const float o = __half2float(__float2half_rn(__uint_as_float(v[i + 1])));
+            if (is_v) {
+                out[i] = __float2half_rn(__uint_as_float(v[i]));
+                out[i + 1] = __float2half_rn(__uint_as_float(v[i + 1]));
+            } else {
+                const int local = (col0 < p.n_q ? col0 : col0 - p.n_q) + i;
+                const float2 cs = p.rope_cs[(size_t)row * half_dim + ((local >> 1) % half_dim)];
+                out[i] = __float2half_rn(__fmaf_rn(cs.x, e, -__fmul_rn(cs.y, o)));
+                out[i + 1] = __float2half_rn(__fmaf_rn(cs.y, e, __fmul_rn(cs.x, o)));
+            }
+        }
+        __half *dstp = nullptr;
+        if (col0 < p.n_q) dstp = p.c + (size_t)row * p.n_q + col0;
+        else if (pos >= 0 && pos < p.max_pos)
+            dstp = (is_v ? p.v_cache + cache_row * p.n_kv + (col0 - p.n_q - p.n_kv)
+                         : p.k_cache + cache_row * p.n_kv + (col0 - p.n_q));
+        if (dstp) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) reinterpret_cast<uint4 *>(dstp)[i] = reinterpret_cast<const uint4 *>(out)[i];
+        }
+    }
+}
+
 // [rows][k] FP16 row-major as a 2-D tensor map with a 64 x box_rows box and 128-byte swizzle (gemm_tc.cu).
 int make_map(CUtensorMap *map, const void *base, int rows, int k, int box_rows);
 
@@ -134,20 +204,15 @@ int make_map_3d(CUtensorMap *map, const void *base, int d0, int d1, int d2, size
 // pdl: programmatic stream serialization at any m (the weights must not be the previous kernel's output).
 int launch_gemm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream);
 
+// What every path of launch_gemm passes on of its arguments (gemm_tc.cu).
+int fill_gemm_params(GemmParams &p, const LlmbGemmArgs *a, int rows_per_seq);
+
+// The path for grids of many tiles (gemm_wide.cu), and whether it takes this one.
+bool gemm_wide_takes(const LlmbGemmArgs *a);
+int launch_gemm_wide(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream);
+
 // Its small-M path (gemm_smallm.cu): m <= 32 rows.
 int launch_gemm_smallm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream);
-
-// Position and cache row of row `row` of a ROPE_KV launch.
-__device__ __forceinline__ int kv_position(const GemmParams &p, int row, size_t &cache_row) {
-    if (p.row_pos) {
-        const int pos = __ldg(p.row_pos + row);
-        cache_row = (size_t)row * (size_t)p.seq_stride + (size_t)pos;
-        return pos;
-    }
-    const int seq = row / p.rows_per_seq, pos = p.pos0 + (row - seq * p.rows_per_seq);
-    cache_row = (size_t)seq * (size_t)p.seq_stride + (size_t)pos;
-    return pos;
-}
 
 // Causal attention of `len` new rows of each of n_seqs sequences (attn_prefill.cu); the caches of consecutive
 // sequences are seq_stride elements apart, q and out are [n_seqs * len][n_q_heads * head_dim].

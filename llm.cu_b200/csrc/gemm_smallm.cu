@@ -337,17 +337,7 @@ int launch_gemm_smallm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaSt
     if ((rc = make_map(&mw2, dual ? a->b2 : a->b, a->n, a->k, kBM))) return rc;
     if ((rc = make_map(&mx, a->a, a->m, a->k, kNX))) return rc;
     GemmParams p = {};
-    p.c = reinterpret_cast<__half *>(a->c);
-    p.rope_cs = reinterpret_cast<const float2 *>(a->rope_cs);
-    p.k_cache = reinterpret_cast<__half *>(a->k_cache);
-    p.v_cache = reinterpret_cast<__half *>(a->v_cache);
-    p.status = device_status_ptr();
-    if (!p.status) return LLMB_ERR_CUDA;
-    p.M = a->m; p.N = a->n; p.K = a->k; p.epilogue = a->epilogue;
-    p.n_q = a->n_q; p.n_kv = a->n_kv; p.head_dim = a->head_dim; p.pos0 = a->pos0; p.max_pos = a->max_pos;
-    p.row_pos = a->row_pos;
-    p.seq_stride = a->seq_stride;
-    p.rows_per_seq = rows_per_seq > 0 ? rows_per_seq : a->m;
+    if ((rc = fill_gemm_params(p, a, rows_per_seq))) return rc;
     p.trace = reinterpret_cast<unsigned long long *>(a->trace);
     p.tp_seq = nullptr;
     if (a->epilogue == LLMB_EPI_TP_SCATTER) {

@@ -207,60 +207,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 tmem_ld32(taddr, v);
                 if (DUAL) tmem_ld32(taddr + kBN, u);
             }
-            if (!row_ok) continue;
-            const int col0 = n0 + c * 32;
-            __align__(16) __half out[32];
-            if (DUAL) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) out[i] = __float2half_rn(silu_gemm(__uint_as_float(v[i])) * __uint_as_float(u[i]));
-                uint4 *dst = reinterpret_cast<uint4 *>(p.c + (size_t)row * p.N + col0);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) dst[i] = reinterpret_cast<const uint4 *>(out)[i];
-            } else if (p.epilogue == LLMB_EPI_STORE) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) out[i] = __float2half_rn(__uint_as_float(v[i]));
-                uint4 *dst = reinterpret_cast<uint4 *>(p.c + (size_t)row * p.N + col0);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) dst[i] = reinterpret_cast<const uint4 *>(out)[i];
-            } else if (p.epilogue == LLMB_EPI_RESIDUAL) {
-                uint4 *dst = reinterpret_cast<uint4 *>(p.c + (size_t)row * p.N + col0);
-                __align__(16) __half res[32];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) reinterpret_cast<uint4 *>(res)[i] = dst[i];
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    out[i] = __float2half_rn(__half2float(__float2half_rn(__uint_as_float(v[i]))) + __half2float(res[i]));
-#pragma unroll
-                for (int i = 0; i < 4; ++i) dst[i] = reinterpret_cast<const uint4 *>(out)[i];
-            } else {  // LLMB_EPI_ROPE_KV
-                size_t cache_row;
-                const int pos = kv_position(p, row, cache_row);
-                const int half_dim = p.head_dim >> 1;
-                const bool is_v = col0 >= p.n_q + p.n_kv;
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    const float e = __half2float(__float2half_rn(__uint_as_float(v[i])));
-                    const float o = __half2float(__float2half_rn(__uint_as_float(v[i + 1])));
-                    if (is_v) {
-                        out[i] = __float2half_rn(__uint_as_float(v[i]));
-                        out[i + 1] = __float2half_rn(__uint_as_float(v[i + 1]));
-                    } else {
-                        const int local = (col0 < p.n_q ? col0 : col0 - p.n_q) + i;
-                        const float2 cs = p.rope_cs[(size_t)row * half_dim + ((local >> 1) % half_dim)];
-                        out[i] = __float2half_rn(__fmaf_rn(cs.x, e, -__fmul_rn(cs.y, o)));
-                        out[i + 1] = __float2half_rn(__fmaf_rn(cs.y, e, __fmul_rn(cs.x, o)));
-                    }
-                }
-                __half *dstp = nullptr;
-                if (col0 < p.n_q) dstp = p.c + (size_t)row * p.n_q + col0;
-                else if (pos >= 0 && pos < p.max_pos)
-                    dstp = (is_v ? p.v_cache + cache_row * p.n_kv + (col0 - p.n_q - p.n_kv)
-                                 : p.k_cache + cache_row * p.n_kv + (col0 - p.n_q));
-                if (dstp) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) reinterpret_cast<uint4 *>(dstp)[i] = reinterpret_cast<const uint4 *>(out)[i];
-                }
-            }
+            if (row_ok) finish_cols<DUAL>(p, row, n0 + c * 32, v, u);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -328,6 +275,22 @@ int make_map_3d(CUtensorMap *map, const void *base, int d0, int d1, int d2, size
     return LLMB_OK;
 }
 
+int fill_gemm_params(GemmParams &p, const LlmbGemmArgs *a, int rows_per_seq) {
+    p.c = reinterpret_cast<__half *>(a->c);
+    p.rope_cs = reinterpret_cast<const float2 *>(a->rope_cs);
+    p.k_cache = reinterpret_cast<__half *>(a->k_cache);
+    p.v_cache = reinterpret_cast<__half *>(a->v_cache);
+    p.status = device_status_ptr();
+    if (!p.status) return LLMB_ERR_CUDA;
+    p.M = a->m; p.N = a->n; p.K = a->k; p.epilogue = a->epilogue;
+    p.n_q = a->n_q; p.n_kv = a->n_kv; p.head_dim = a->head_dim; p.pos0 = a->pos0; p.max_pos = a->max_pos;
+    p.row_pos = a->row_pos;
+    p.seq_stride = a->seq_stride;
+    p.rows_per_seq = rows_per_seq > 0 ? rows_per_seq : a->m;
+    p.splits = 1;
+    return LLMB_OK;
+}
+
 }  // namespace llmb
 
 extern "C" int llmb_gemm_f16(const LlmbGemmArgs *a, llmb_stream_t stream_) {
@@ -343,7 +306,7 @@ int llmb::launch_gemm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStr
         set_last_error("llmb_gemm_f16: n must be a multiple of 128 and k a multiple of 64");
         return LLMB_ERR_UNSUPPORTED;
     }
-    if (a->epilogue == LLMB_EPI_TP_SCATTER && !small_m) {
+    if (a->epilogue == LLMB_EPI_TP_SCATTER && (a->m > 32 || a->tile_n != 0)) {
         set_last_error("llmb_gemm_f16: LLMB_EPI_TP_SCATTER needs m <= 32");
         return LLMB_ERR_UNSUPPORTED;
     }
@@ -358,6 +321,7 @@ int llmb::launch_gemm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStr
     }
     // A handful of rows (batched decode): the weight-streaming kernel with the operands swapped
     if (small_m) return launch_gemm_smallm(a, rows_per_seq, pdl, stream);
+    if (gemm_wide_takes(a)) return launch_gemm_wide(a, rows_per_seq, pdl, stream);
     // Small grids: with a workspace, 128-wide tiles and K split across CTAs until the SMs are covered
     // (every CTA then streams its own weights and only its slice of the activations); without one, the
     // widest tile that still gives every SM a CTA.
@@ -380,20 +344,9 @@ int llmb::launch_gemm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStr
     if ((rc = make_map(&mb, a->b, a->n, a->k, bn))) return rc;
     if ((rc = make_map(&mb2, dual ? a->b2 : a->b, a->n, a->k, bn))) return rc;
     GemmParams p = {};
-    p.c = reinterpret_cast<__half *>(a->c);
-    p.rope_cs = reinterpret_cast<const float2 *>(a->rope_cs);
-    p.k_cache = reinterpret_cast<__half *>(a->k_cache);
-    p.v_cache = reinterpret_cast<__half *>(a->v_cache);
-    p.status = device_status_ptr();
-    if (!p.status) return LLMB_ERR_CUDA;
-    p.M = a->m; p.N = a->n; p.K = a->k; p.epilogue = a->epilogue;
-    p.n_q = a->n_q; p.n_kv = a->n_kv; p.head_dim = a->head_dim; p.pos0 = a->pos0; p.max_pos = a->max_pos;
-    p.row_pos = a->row_pos;
-    p.seq_stride = a->seq_stride;
-    p.rows_per_seq = rows_per_seq > 0 ? rows_per_seq : a->m;
+    if ((rc = fill_gemm_params(p, a, rows_per_seq))) return rc;
     dim3 grid(m_tiles, a->n / bn);
     const int tiles = (int)(grid.x * grid.y), k_tiles = a->k / kBK;
-    p.splits = 1;
     if (have_ws && tiles * 2 <= sms && tiles <= 1024) {
         int splits = sms / tiles;
         if (splits > 8) splits = 8;
