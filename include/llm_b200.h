@@ -210,8 +210,8 @@ int llmb_advance_pos(int32_t *d_pos, int use_pdl, llmb_stream_t stream);
 /*                      k, v -> cache row pos0 + row                     (inference.cu:640-695) */
 /*   LLMB_EPI_SWIGLU    c = half(SiLU(A.b^T) * (A.b2^T)), accumulators not rounded  (:515)     */
 /* n must be a multiple of 128, k of 64; a, b, c 16-byte aligned; m is free (rows past m are   */
-/* zero-filled on load and never stored).  With m <= 32 (and tile_n 0) the launch is a weight  */
-/* stream: the weight tile is the 128-row MMA operand, the m rows the 32-column one, K is split */
+/* zero-filled on load and never stored).  With m <= 128 (and tile_n 0) the launch is a weight  */
+/* stream: the weight tile is the 128-row MMA operand, the m rows the other one, K is split     */
 /* until two CTAs per SM stream weights (the slices of a tile are one thread-block cluster and   */
 /* add their partial sums through distributed shared memory: no workspace), bound by HBM like   */
 /* llmb_gemv_f16.                                                                                */
@@ -230,7 +230,7 @@ typedef struct {
     int pos0;              /* cache row of A's row 0 */
     int max_pos;
     int tile_n;            /* output columns per CTA: 0 = the widest of 128/64/32 that fills the SMs */
-    void *workspace;       /* m > 32 only. Optional, 16-byte aligned, its first 4096 bytes zero before the first use (the */
+    void *workspace;       /* m > 128 only. Optional, 16-byte aligned, its first 4096 bytes zero before the first use (the */
     size_t workspace_bytes;/* kernel leaves them zero): lets a launch with few output tiles split K across     */
                            /* CTAs; partial sums are added in slice order.  One launch at a time per workspace; */
                            /* 4096 + SMs * 131072 bytes always suffice.                                        */

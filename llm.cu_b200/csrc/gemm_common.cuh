@@ -29,6 +29,7 @@ struct GemmParams {
     const int *row_pos;  // ROPE_KV, batched decode: cache position of each row; row r belongs to sequence r
     long long seq_stride;  // cache rows between consecutive sequences
     int rows_per_seq;      // ROPE_KV without row_pos: row r = position pos0 + r % rows_per_seq of sequence r / rows_per_seq
+    int nx;      // small-M kernel: columns of the MMA, the activation rows rounded up to 32
     int stages;  // ring depth of this launch (<= kGemmMaxStages)
     // split-K: blockIdx.z takes a slice of K, partial accumulators meet in the workspace and the last
     // CTA of a tile to arrive adds them in slice order and runs the epilogue
@@ -211,7 +212,8 @@ int fill_gemm_params(GemmParams &p, const LlmbGemmArgs *a, int rows_per_seq);
 bool gemm_wide_takes(const LlmbGemmArgs *a);
 int launch_gemm_wide(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream);
 
-// Its small-M path (gemm_smallm.cu): m <= 32 rows.
+// Its small-M path (gemm_smallm.cu): m <= kSmallM rows.
+constexpr int kSmallM = 128;
 int launch_gemm_smallm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream);
 
 // Causal attention of `len` new rows of each of n_seqs sequences (attn_prefill.cu); the caches of consecutive

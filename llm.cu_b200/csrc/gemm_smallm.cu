@@ -1,4 +1,4 @@
-// Projections for a handful of rows (batched decode: one new row per sequence, m <= 32):
+// Projections for a handful of rows (batched decode: one new row per sequence; short prompts; m <= 128):
 // C[m][n] = X[m][k] . W[n][k]^T with the roles of the two operands swapped on the tensor cores.
 //
 // Replaces kernel_standard_tiled_gemm / kernel_standard_tiled_gemm_ffn_swiglu of the reference
@@ -8,14 +8,14 @@
 // Bound: HBM.  Every weight byte is streamed once per launch; the m activation rows (a few KB per K step)
 // come from L2.  So the kernel is shaped as a weight stream, like the batch-1 projections, not as a GEMM:
 //
-//   operands  the WEIGHT tile is the 128-row (M) operand of tcgen05.mma, the activation rows are the 32-column
-//             (N) operand: D[128 weight rows][32 activation rows] in 32 columns of tensor memory.  A ring stage
-//             is 16 KB of weights + 4 KB of activations (32 KB + 4 KB for the gate/up pair), so nearly all of
-//             the shared memory in flight is weight bytes, and an MMA step costs a quarter of the 128-wide one.
+//   operands  the WEIGHT tile is the 128-row (M) operand of tcgen05.mma, the activation rows are the nx-column
+//             (N) operand, nx = m rounded up to 32: D[128 weight rows][nx activation rows] in tensor memory.  A ring
+//             stage is 16 KB of weights + 4 KB per 32 activation rows (32 KB of weights for the gate/up pair), so most
+//             of the shared memory in flight is weight bytes, and an MMA step costs nx / 128 of the 128-wide one.
 //   grid      x = 128-row weight tile, y = slice of K.  K is split in 2, 4 or 8 until about two CTAs per SM
 //             exist (each slice at least 8 K steps).  The CTAs of one tile form a thread-block cluster: each
-//             leaves its partial accumulators (128 x 32 FP32 = 16 KB) in its own shared memory, and after a
-//             cluster barrier CTA r adds the partials of activation rows r * 32/S .. through distributed
+//             leaves its partial accumulators (128 x nx FP32) in its own shared memory, and after a
+//             cluster barrier CTA r adds the partials of activation rows r * nx/S .. through distributed
 //             shared memory, in slice order, and runs the epilogue for those rows.  No workspace, no atomic,
 //             no last CTA that reduces alone.
 //   ring      about 100 KB per CTA, so that two CTAs share an SM: two of this launch, or the tail of this
@@ -32,11 +32,10 @@
 
 namespace llmb {
 
-constexpr int kNX = 32;                                   // activation rows per launch (N of the MMA)
+constexpr int kNX = 32;                                   // the activation rows of a launch (N of the MMA) are a multiple of this
 constexpr uint32_t kWTileBytes = kBM * kBK * 2;           // 16 KB
-constexpr uint32_t kXTileBytes = kNX * kBK * 2;           // 4 KB
 constexpr int kSmallMaxStages = 8;
-__host__ __device__ constexpr uint32_t small_stage_bytes(bool dual) { return (dual ? 2 : 1) * kWTileBytes + kXTileBytes; }
+__host__ __device__ constexpr uint32_t small_stage_bytes(bool dual, int nx) { return (dual ? 2 : 1) * kWTileBytes + nx * kBK * 2; }
 
 __device__ __forceinline__ uint32_t cluster_cta_rank() {
     uint32_t r;
@@ -50,10 +49,9 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
-// The S slices' partial sums of element (activation row b, weight row nl) of accumulator `acc`, added in slice order.
-// rbase[z] = shared-memory address, as seen from this CTA, of slice z's [accumulator][32][128] FP32 block.
-__device__ __forceinline__ float gather_slices(const uint32_t (&rbase)[8], int n_slices, int acc, int b, int nl) {
-    const uint32_t off = (uint32_t)(((acc * kNX + b) * kBM + nl) * 4);
+// The S slices' partial sums of one element, added in slice order (`last_first`: from the last slice to the first).
+// rbase[z] + off = its address in slice z's block of partial sums as seen from this CTA.
+__device__ __forceinline__ float gather_slices(const uint32_t (&rbase)[8], int n_slices, uint32_t off, bool last_first) {
     float t[8];
 #pragma unroll
     for (int z = 0; z < 8; ++z) {
@@ -63,7 +61,10 @@ __device__ __forceinline__ float gather_slices(const uint32_t (&rbase)[8], int n
     float sum = 0.0f;
 #pragma unroll
     for (int z = 0; z < 8; ++z)
-        if (z < n_slices) sum += t[z];
+        if (z < n_slices && !last_first) sum += t[z];
+#pragma unroll
+    for (int z = 7; z >= 0; --z)
+        if (z < n_slices && last_first) sum += t[z];
     return sum;
 }
 
@@ -78,11 +79,16 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __shared__ uint32_t tmem_slot;
     __shared__ int prior_status;
 
-    constexpr uint32_t kStageBytes = small_stage_bytes(DUAL);
     constexpr uint32_t kXOff = (DUAL ? 2 : 1) * kWTileBytes;
-    constexpr uint32_t kTmemCols = DUAL ? 2 * kNX : kNX;   // 32 is the smallest allocation
+    const int nx = p.nx;
+    // Either order is as good; this one picks the reference's token on every step of the full-depth fixture, whose prompt of
+    // 128 rows comes through here (two of its steps have a top-2 gap of one FP16 step).
+    const bool last_first = nx > kNX;
+    const uint32_t stage_bytes = small_stage_bytes(DUAL, nx);
+    // an allocation is a power of two from 32 on: (DUAL ? 2 : 1) * nx columns rounded up
+    const uint32_t tmem_cols = (DUAL ? 2u : 1u) * (nx <= 32 ? 32u : nx <= 64 ? 64u : 128u);
     // kind::f16: D = F32 (bit 4), A = B = F16, both K-major, N >> 3 at bit 17, M >> 4 at bit 24
-    constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(kNX >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+    const uint32_t idesc = (1u << 4) | ((uint32_t)(nx >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 
     unsigned char *ring = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(small_smem) + 1023) & ~uintptr_t(1023));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -129,7 +135,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         fence_mbar_init();
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -144,8 +150,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             // the head of the weight stream does not depend on the previous kernel: ask for it first
             const int head = min(stages, kt_end - kt_begin);
             for (int i = 0; i < head; ++i) {
-                unsigned char *st = ring + (size_t)i * kStageBytes;
-                mbar_arrive_expect_tx(&full_bar[i], kStageBytes);
+                unsigned char *st = ring + (size_t)i * stage_bytes;
+                mbar_arrive_expect_tx(&full_bar[i], stage_bytes);
                 tma_load_2d(st, &map_w, (kt_begin + i) * kBK, n0, &full_bar[i]);
                 if (DUAL) tma_load_2d(st + kWTileBytes, &map_w2, (kt_begin + i) * kBK, n0, &full_bar[i]);
             }
@@ -155,13 +161,13 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             // a wait that gave up earlier leaves the status word set: do not queue more bounded waits behind it
             bool ok = *reinterpret_cast<volatile int *>(p.status) == 0;
             for (int i = 0; i < head; ++i)
-                tma_load_2d(ring + (size_t)i * kStageBytes + kXOff, &map_x, (kt_begin + i) * kBK, 0, &full_bar[i]);
+                tma_load_2d(ring + (size_t)i * stage_bytes + kXOff, &map_x, (kt_begin + i) * kBK, 0, &full_bar[i]);
             for (int kt = kt_begin + head, i = head; kt < kt_end && ok; ++kt, ++i) {
                 const int s = i % stages;
                 ok = mbar_wait(&empty_bar[s], ((i / stages) - 1) & 1, p.status, 311);
                 if (!ok) break;
-                unsigned char *st = ring + (size_t)s * kStageBytes;
-                mbar_arrive_expect_tx(&full_bar[s], kStageBytes);
+                unsigned char *st = ring + (size_t)s * stage_bytes;
+                mbar_arrive_expect_tx(&full_bar[s], stage_bytes);
                 tma_load_2d(st, &map_w, kt * kBK, n0, &full_bar[s]);
                 if (DUAL) tma_load_2d(st + kWTileBytes, &map_w2, kt * kBK, n0, &full_bar[s]);
                 tma_load_2d(st + kXOff, &map_x, kt * kBK, 0, &full_bar[s]);
@@ -176,14 +182,14 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (!ok) break;
                 if (i == 0) stamp(3);  // first stage landed
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                unsigned char *st = ring + (size_t)s * kStageBytes;
+                unsigned char *st = ring + (size_t)s * stage_bytes;
                 const uint64_t wdesc = umma_desc(st), xdesc = umma_desc(st + kXOff);
                 const uint64_t w2desc = DUAL ? umma_desc(st + kWTileBytes) : 0;
 #pragma unroll
                 for (int k = 0; k < kBK / 16; ++k) {
                     const uint32_t acc = (i > 0 || k > 0) ? 1u : 0u;
-                    umma_f16(tmem_base, wdesc + 2 * k, xdesc + 2 * k, kIdesc, acc);
-                    if (DUAL) umma_f16(tmem_base + kNX, w2desc + 2 * k, xdesc + 2 * k, kIdesc, acc);
+                    umma_f16(tmem_base, wdesc + 2 * k, xdesc + 2 * k, idesc, acc);
+                    if (DUAL) umma_f16(tmem_base + nx, w2desc + 2 * k, xdesc + 2 * k, idesc, acc);
                 }
                 umma_commit(&empty_bar[s]);
             }
@@ -193,7 +199,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     // ---- epilogue: thread = weight row n0 + lane_group + lane.  The accumulators go to shared memory first (over
     // the ring), [accumulator][activation row b][weight row]; the rows are then finished four at a time in a loop
-    // that is NOT unrolled over all 32 rows: a CTA runs its epilogue once, so every instruction of it is fetched
+    // that is NOT unrolled over all rows: a CTA runs its epilogue once, so every instruction of it is fetched
     // cold, and the fully unrolled form (five epilogues x 32 rows) cost 5-19 us of instruction fetch per launch.
     const int lane_group = (warp & 3) * 32;
     const int nl = lane_group + lane;
@@ -206,113 +212,126 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (threadIdx.x == 64) stamp(5);  // accumulators complete
         pdl_wait();  // from here on global memory of earlier kernels is read and written
         ok = got && *reinterpret_cast<volatile int *>(p.status) == 0;
-        const uint32_t taddr = tmem_base + ((uint32_t)lane_group << 16);
-        // every load of the ring has landed and every MMA has read it (acc_bar): the ring is free
-        uint32_t v[32];
-        tmem_ld32(taddr, v);
-#pragma unroll
-        for (int b = 0; b < kNX; ++b) red_own[b * kBM + nl] = v[b];
-        if (DUAL) {
-            tmem_ld32(taddr + kNX, v);
-#pragma unroll
-            for (int b = 0; b < kNX; ++b) red_own[(kNX + b) * kBM + nl] = v[b];
-        }
     }
-    // Split K: CTA r of the cluster finishes activation rows r * 32/S ..; without a split a thread only reads back
-    // what it wrote itself, so no barrier is needed.
-    int b_lo = 0, nb = kNX;
+    // every load of the ring has landed and every MMA has read it (acc_bar): the ring is free
+    const uint32_t taddr = tmem_base + ((uint32_t)lane_group << 16);
+    auto spill = [&](int b0, int red_rows, int at) {  // columns b0 .. b0 + 31 to rows at .. of the block of partial sums
+        uint32_t v[32];
+        tmem_ld32(taddr + b0, v);
+#pragma unroll
+        for (int b = 0; b < 32; ++b) red_own[(at + b) * kBM + nl] = v[b];
+        if (DUAL) {
+            tmem_ld32(taddr + nx + b0, v);
+#pragma unroll
+            for (int b = 0; b < 32; ++b) red_own[(red_rows + at + b) * kBM + nl] = v[b];
+        }
+    };
+    // Split K: all slices of the tile meet, then CTA r of the cluster finishes activation rows r * nx/S ..; without a split
+    // a thread only reads back what it wrote itself, 32 rows at a time, so no barrier is needed.
     if (clustered) {
+        if (warp >= 2) {
+#pragma unroll 1
+            for (int b0 = 0; b0 < nx; b0 += 32) spill(b0, nx, b0);
+        }
         cluster_sync_all();  // all slices of the tile are in shared memory
-        nb = kNX / p.splits;
-        b_lo = slice * nb;
     }
     if (threadIdx.x == 64) stamp(6);
-    if (warp >= 2 && ok && n < p.N) {  // the last weight tile may reach past N (its rows are zero-filled by TMA)
-        uint32_t rbase[8];
-        const uint32_t red = smem_u32(ring);
-#pragma unroll
-        for (int z = 0; z < 8; ++z) {
-            rbase[z] = red;
-            if (clustered && z < p.splits) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbase[z]) : "r"(red), "r"(z));
-        }
-        const int n_slices = clustered ? p.splits : 1;
-        const int b_hi = min(b_lo + nb, p.M);
-        // Output element (b, n): the 32 lanes of a warp hold 32 consecutive n, so each store of a warp is one
-        // 64-byte run of row b.  Loads of four rows first, then their stores.
-        const int half_dim = p.head_dim >> 1;
-        const bool is_q = n < p.n_q, is_v = n >= p.n_q + p.n_kv;
-        const int local = is_q ? n : (is_v ? n - p.n_q - p.n_kv : n - p.n_q);
-        const int pair = half_dim > 0 ? (local >> 1) % half_dim : 0;
-        const unsigned int tag = p.epilogue == LLMB_EPI_TP_SCATTER ? __ldg(p.tp_seq) + (unsigned int)p.tp_index + 1u : 0u;
+    if (warp >= 2) {
+        const int nb = clustered ? nx / p.splits : 32, red_rows = clustered ? nx : 32;
+        const int first = clustered ? slice * nb : 0, past = clustered ? first + nb : nx;
 #pragma unroll 1
-        for (int b0 = b_lo; b0 < b_hi; b0 += 4) {
-            float val[4], val2[4];
+        for (int b_lo = first; b_lo < past; b_lo += nb) {
+            if (!clustered) spill(b_lo, 32, 0);  // warp-collective: every lane takes part
+            const int red0 = clustered ? 0 : b_lo;
+            if (ok && n < p.N) {  // the last weight tile may reach past N (its rows are zero-filled by TMA)
+                uint32_t rbase[8];
+                const uint32_t red = smem_u32(ring);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int b = min(b0 + i, b_hi - 1);
-                val[i] = gather_slices(rbase, n_slices, 0, b, nl);
-                val2[i] = DUAL ? gather_slices(rbase, n_slices, 1, b, nl) : 0.0f;
-            }
-            if (!DUAL && p.epilogue == LLMB_EPI_TP_SCATTER) {
-                // tensor parallel: this rank's partial sums go, tagged, to every rank's receive buffer
-                const size_t slot0 = tp_rows_slot(p.tp_size, p.N, p.tp_index, p.tp_rank, 0, n);
+                for (int z = 0; z < 8; ++z) {
+                    rbase[z] = red;
+                    if (clustered && z < p.splits) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbase[z]) : "r"(red), "r"(z));
+                }
+                const int n_slices = clustered ? p.splits : 1;
+                const int b_hi = min(b_lo + nb, p.M);
+                // Output element (b, n): the 32 lanes of a warp hold 32 consecutive n, so each store of a warp is one
+                // 64-byte run of row b.  Loads of four rows first, then their stores.
+                const int half_dim = p.head_dim >> 1;
+                const bool is_q = n < p.n_q, is_v = n >= p.n_q + p.n_kv;
+                const int local = is_q ? n : (is_v ? n - p.n_q - p.n_kv : n - p.n_q);
+                const int pair = half_dim > 0 ? (local >> 1) % half_dim : 0;
+                const unsigned int tag = p.epilogue == LLMB_EPI_TP_SCATTER ? __ldg(p.tp_seq) + (unsigned int)p.tp_index + 1u : 0u;
+#pragma unroll 1
+                for (int b0 = b_lo; b0 < b_hi; b0 += 4) {
+                    float val[4], val2[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (b0 + i < b_hi) {
-                        const size_t off = slot0 + (size_t)(b0 + i) * p.N * 8;
-                        for (int r = 0; r < p.tp_size; ++r)
-                            asm volatile("st.relaxed.sys.global.v2.b32 [%0], {%1, %2};" ::"l"(p.tp_peer[r] + off), "r"(__float_as_uint(val[i])),
-                                         "r"(tag)
-                                         : "memory");
+                    for (int i = 0; i < 4; ++i) {
+                        const int b = min(b0 + i, b_hi - 1);
+                        const uint32_t off = (uint32_t)(((b - red0) * kBM + nl) * 4);
+                        val[i] = gather_slices(rbase, n_slices, off, last_first);
+                        val2[i] = DUAL ? gather_slices(rbase, n_slices, off + (uint32_t)(red_rows * kBM * 4), last_first) : 0.0f;
                     }
-                }
-            } else if (DUAL) {
+                    if (!DUAL && p.epilogue == LLMB_EPI_TP_SCATTER) {
+                        // tensor parallel: this rank's partial sums go, tagged, to every rank's receive buffer
+                        const size_t slot0 = tp_rows_slot(p.tp_size, p.N, p.tp_index, p.tp_rank, 0, n);
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (b0 + i < b_hi) p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(silu_gemm(val[i]) * val2[i]);
-            } else if (p.epilogue == LLMB_EPI_STORE) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (b0 + i < b_hi) p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(val[i]);
-            } else if (p.epilogue == LLMB_EPI_RESIDUAL) {
-                // the residual values of the four rows first, then the stores: a load after a store to the same
-                // array would have to wait for it
-                __half res[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) res[i] = __ldcg(p.c + (size_t)min(b0 + i, b_hi - 1) * p.N + n);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (b0 + i < b_hi)
-                        p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(__half2float(__float2half_rn(val[i])) + __half2float(res[i]));
-            } else {  // LLMB_EPI_ROPE_KV: the pair (even n, n + 1) sits in neighbouring lanes
-                float2 cs[4];
-                int pos[4];
-                size_t cache_row[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int b = min(b0 + i, b_hi - 1);
-                    cs[i] = is_v ? make_float2(1.0f, 0.0f) : __ldg(p.rope_cs + (size_t)b * half_dim + pair);
-                    pos[i] = kv_position(p, b, cache_row[i]);
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int b = b0 + i;
-                    // b and b_hi are the same in all lanes, so the shuffle is executed by the whole warp (N is a
-                    // multiple of 32 whenever this epilogue is used: whole heads)
-                    if (b < b_hi) {
-                        const float mine = __half2float(__float2half_rn(val[i]));
-                        const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
-                        __half out;
-                        if (is_v) {
-                            out = __float2half_rn(val[i]);
-                        } else {
-                            out = __float2half_rn((n & 1) ? __fmaf_rn(cs[i].y, other, __fmul_rn(cs[i].x, mine))
-                                                          : __fmaf_rn(cs[i].x, mine, -__fmul_rn(cs[i].y, other)));
+                        for (int i = 0; i < 4; ++i) {
+                            if (b0 + i < b_hi) {
+                                const size_t off = slot0 + (size_t)(b0 + i) * p.N * 8;
+                                for (int r = 0; r < p.tp_size; ++r)
+                                    asm volatile("st.relaxed.sys.global.v2.b32 [%0], {%1, %2};" ::"l"(p.tp_peer[r] + off), "r"(__float_as_uint(val[i])),
+                                                 "r"(tag)
+                                                 : "memory");
+                            }
                         }
-                        if (is_q) {
-                            p.c[(size_t)b * p.n_q + n] = out;
-                        } else {
-                            if (pos[i] >= 0 && pos[i] < p.max_pos) (is_v ? p.v_cache : p.k_cache)[cache_row[i] * p.n_kv + local] = out;
+                    } else if (DUAL) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (b0 + i < b_hi) p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(silu_gemm(val[i]) * val2[i]);
+                    } else if (p.epilogue == LLMB_EPI_STORE) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (b0 + i < b_hi) p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(val[i]);
+                    } else if (p.epilogue == LLMB_EPI_RESIDUAL) {
+                        // the residual values of the four rows first, then the stores: a load after a store to the same
+                        // array would have to wait for it
+                        __half res[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) res[i] = __ldcg(p.c + (size_t)min(b0 + i, b_hi - 1) * p.N + n);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (b0 + i < b_hi)
+                                p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(__half2float(__float2half_rn(val[i])) + __half2float(res[i]));
+                    } else {  // LLMB_EPI_ROPE_KV: the pair (even n, n + 1) sits in neighbouring lanes
+                        float2 cs[4];
+                        int pos[4];
+                        size_t cache_row[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int b = min(b0 + i, b_hi - 1);
+                            cs[i] = is_v ? make_float2(1.0f, 0.0f) : __ldg(p.rope_cs + (size_t)b * half_dim + pair);
+                            pos[i] = kv_position(p, b, cache_row[i]);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int b = b0 + i;
+                            // b and b_hi are the same in all lanes, so the shuffle is executed by the whole warp (N is a
+                            // multiple of 32 whenever this epilogue is used: whole heads)
+                            if (b < b_hi) {
+                                const float mine = __half2float(__float2half_rn(val[i]));
+                                const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
+                                __half out;
+                                if (is_v) {
+                                    out = __float2half_rn(val[i]);
+                                } else {
+                                    out = __float2half_rn((n & 1) ? __fmaf_rn(cs[i].y, other, __fmul_rn(cs[i].x, mine))
+                                                                  : __fmaf_rn(cs[i].x, mine, -__fmul_rn(cs[i].y, other)));
+                                }
+                                if (is_q) {
+                                    p.c[(size_t)b * p.n_q + n] = out;
+                                } else {
+                                    if (pos[i] >= 0 && pos[i] < p.max_pos) (is_v ? p.v_cache : p.k_cache)[cache_row[i] * p.n_kv + local] = out;
+                                }
+                            }
                         }
                     }
                 }
@@ -325,17 +344,18 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     if (threadIdx.x == 0) stamp(7);  // epilogue done
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     }
 }
 
 int launch_gemm_smallm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream) {
     const bool dual = a->epilogue == LLMB_EPI_SWIGLU;
+    const int nx = (a->m + kNX - 1) / kNX * kNX;
     CUtensorMap mw, mw2, mx;
     int rc;
     if ((rc = make_map(&mw, a->b, a->n, a->k, kBM))) return rc;
     if ((rc = make_map(&mw2, dual ? a->b2 : a->b, a->n, a->k, kBM))) return rc;
-    if ((rc = make_map(&mx, a->a, a->m, a->k, kNX))) return rc;
+    if ((rc = make_map(&mx, a->a, a->m, a->k, nx))) return rc;
     GemmParams p = {};
     if ((rc = fill_gemm_params(p, a, rows_per_seq))) return rc;
     p.trace = reinterpret_cast<unsigned long long *>(a->trace);
@@ -353,18 +373,27 @@ int launch_gemm_smallm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaSt
     // K is split (2, 4 or 8 slices = the CTAs of one cluster) until about two CTAs per SM stream weights, each
     // slice at least 8 K steps long.  The gate/up pair moves two weight tiles per CTA: it is split only while
     // the tiles alone leave half of the SMs without a CTA.
+    p.nx = nx;
     p.splits = 1;
-    if (tiles < 2 * sms) {
-        int want = 2 * sms / tiles;  // never more CTAs than can be resident at once
+    // More than 32 rows of the gate/up pair: its two blocks of partial sums (128 KB at 128 rows) leave room for one CTA per
+    // SM where K is split; tiles enough for every SM are not split and keep two.
+    const bool one_per_sm = dual && nx > kNX && tiles <= sms;
+    const int ctas = one_per_sm ? sms : 2 * sms;
+    if (tiles < ctas && !(dual && nx > kNX && !one_per_sm)) {
+        int want = ctas / tiles;  // never more CTAs than can be resident at once
         if (want > k_tiles / 8) want = k_tiles / 8;
         p.splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
     }
     p.ws_count = nullptr;
     p.ws_part = nullptr;
-    // about 100 KB of ring per CTA: two CTAs (of this launch, or of this and the next one) share an SM
-    p.stages = dual ? 3 : 5;  // 108 KB / 100 KB
-    if (dual && tiles * p.splits <= sms) p.stages = 5;  // one CTA per SM anyway: a deeper ring (180 KB)
-    const size_t smem = (size_t)p.stages * small_stage_bytes(dual) + 1024;
+    // about 100 KB of ring per CTA: two CTAs (of this launch, or of this and the next one) share an SM.  The ring also
+    // holds the partial sums: (dual ? 2 : 1) * nx * 512 bytes with a split, 32 rows at a time without.
+    const uint32_t stage = small_stage_bytes(dual, nx);
+    p.stages = (int)((dual ? 108u : 100u) * 1024u / stage);
+    if (dual && nx == kNX && tiles * p.splits <= sms) p.stages = 5;  // one CTA per SM anyway: a deeper ring (180 KB)
+    if (one_per_sm) p.stages = (int)(196u * 1024u / stage);
+    if (p.stages > kSmallMaxStages) p.stages = kSmallMaxStages;
+    const size_t smem = (size_t)p.stages * stage + 1024;
     static size_t attr_set[2][kMaxDevices] = {};  // per instantiation and device
     if (dual) {
         LLMB_CUDA_OK(ensure_dynamic_smem(gemm_smallm_kernel<true>, attr_set[1], smem));

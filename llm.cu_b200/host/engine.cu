@@ -483,14 +483,14 @@ int row_parallel_projection(Engine *e, const void *a, const void *w, int m, int 
     if (e->tp_size > 1) {
         LlmbGemmArgs g = small_gemm(e, a, w, nullptr, m, e->d, k, LLMB_EPI_TP_SCATTER);
         g.tp_index = xi;
-        if ((rc = llmb_gemm_f16(&g, e->stream))) return rc;
+        if ((rc = launch_gemm(&g, 0, true, e->stream))) return rc;
         rc = llmb_tp_gather_rows(e->exchange, e->tp_size, xi, reinterpret_cast<uint16_t *>(e->pf_x), u16(gamma),
                                  reinterpret_cast<uint16_t *>(e->pf_xn), m, e->d, c.eps, e->tag_poll_limit, 1, e->stream);
         ++xi;
         return rc;
     }
     LlmbGemmArgs g = small_gemm(e, a, w, e->pf_x, m, e->d, k, LLMB_EPI_RESIDUAL);
-    if ((rc = llmb_gemm_f16(&g, e->stream))) return rc;
+    if ((rc = launch_gemm(&g, 0, true, e->stream))) return rc;
     if (gamma) rc = llmb_rmsnorm_rows(u16(e->pf_x), u16(gamma), reinterpret_cast<uint16_t *>(e->pf_xn), m, e->d, c.eps, e->stream);
     return rc;
 }
@@ -1133,7 +1133,7 @@ int enqueue_batch_step(Engine *e, const SplitPlan &sp) {
         g.rope_cs = e->pf_rope;
         g.k_cache = u16w(kl); g.v_cache = u16w(vl);
         g.row_pos = e->bt_pos; g.seq_stride = e->max_seq; g.max_pos = e->max_seq;
-        if ((rc = llmb_gemm_f16(&g, s))) return rc;
+        if ((rc = launch_gemm(&g, 0, true, s))) return rc;
         if ((rc = llmb_attn_decode_batch(u16(e->pf_q), u16(kl), u16(vl), e->bt_pos, B, (size_t)e->max_seq, e->nq, e->nkv, e->hd,
                                          sp.n_splits, sp.split_len, u16w(e->pf_attn), e->bt_attn_scratch, 1, s)))
             return rc;
@@ -1142,12 +1142,12 @@ int enqueue_batch_step(Engine *e, const SplitPlan &sp) {
             return rc;
         LlmbGemmArgs f = small_gemm(e, e->pf_xn, L->mlp_gate_proj->d_fp16_tensor, e->pf_h, B, e->ffn, e->d, LLMB_EPI_SWIGLU);
         f.b2 = u16(L->mlp_up_proj->d_fp16_tensor);
-        if ((rc = llmb_gemm_f16(&f, s))) return rc;
+        if ((rc = launch_gemm(&f, 0, true, s))) return rc;
         const void *next_gamma = l + 1 < e->layers ? m->layers[l + 1]->input_layernorm->d_fp16_tensor : m->norm->d_fp16_tensor;
         if ((rc = row_parallel_projection(e, e->pf_h, L->mlp_down_proj->d_fp16_tensor, B, e->ffn, next_gamma, xi))) return rc;
     }
     LlmbGemmArgs lm = small_gemm(e, e->pf_xn, m->lm_head->d_fp16_tensor, e->bt_logits, B, e->vocab, e->d, LLMB_EPI_STORE);
-    if ((rc = llmb_gemm_f16(&lm, s))) return rc;
+    if ((rc = launch_gemm(&lm, 0, true, s))) return rc;
     // greedy token of every sequence -> next step's input; positions advance; history keeps what was sampled
     if (tp) {
         if ((rc = llmb_tp_argmax_rows(e->peers, e->tp_rank, e->tp_size, e->d, xi, u16(e->bt_logits), e->vocab, e->tp_rank * e->vocab, B,

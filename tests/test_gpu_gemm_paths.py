@@ -1,0 +1,86 @@
+"""The two ends of llmb_gemm_f16's dispatch at their edges: the weight-streaming kernel between 33 and 128 rows (column counts
+32 x 2..4, with and without a cluster, gate/up pairs with one or two CTAs per SM) and the persistent 128 x 256 tiles of long
+blocks (ragged rows, a last column tile that is half empty, K shorter than the ring).  Against float64, tolerances as in
+test_gpu_prefill.py."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+from gpu_util import assert_close_fp16, dev, f16, host_u16  # noqa: E402
+from test_gpu_prefill import EPI_RESIDUAL, EPI_ROPE_KV, EPI_STORE, EPI_SWIGLU, gemm, mats, matmul64, tc_tol  # noqa: E402
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _need_gpu():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+SMALL = [(33, 256, 64), (64, 384, 4096), (65, 128, 1024), (96, 1280, 512), (97, 4096, 2048), (128, 512, 4096), (100, 19200, 128), (40, 38144, 64)]
+WIDE = [(2049, 2432, 64), (4096, 1280, 192), (1000, 4864, 320), (300, 12800, 512)]
+
+
+@pytest.mark.parametrize("m,n,k", SMALL + WIDE)
+def test_store_and_residual(pkg, oracle, m, n, k):
+    a, b = mats(oracle, m, n, k, 40)
+    da, db = dev(a), dev(b)
+    out = torch.full((m + 3, n), 0x7BFF, dtype=torch.int16, device="cuda")  # rows past m must stay untouched
+    gemm(pkg, a=da, b=db, c=out, m=m, n=n, k=k, epilogue=EPI_STORE)
+    acc = matmul64(a, b)
+    got = host_u16(out).reshape(m + 3, n)
+    assert_close_fp16(got[:m], acc, what="store", abs_tol=tc_tol(acc, k))
+    assert (got[m:] == 0x7BFF).all()
+    res = oracle.synth_fp16(7, 3, m * n, std=1.0).reshape(m, n)
+    out = dev(res.copy())
+    gemm(pkg, a=da, b=db, c=out, m=m, n=n, k=k, epilogue=EPI_RESIDUAL)
+    want = acc.astype(np.float16).astype(np.float64) + f16(res).astype(np.float64)
+    # half(acc) may sit one FP16 step (|acc| 2^-10) from the product's rounding, and the sum is rounded once more (|want| 2^-10)
+    assert_close_fp16(host_u16(out).reshape(m, n), want, what="residual", max_frac=0.1,
+                      abs_tol=(np.abs(acc) + np.abs(want)) * 2.0 ** -10 + tc_tol(acc, k))
+
+
+@pytest.mark.parametrize("m,n,k", [(33, 128, 512), (64, 640, 1024), (96, 384, 2048), (128, 256, 4096), (128, 19072, 128), (70, 19200, 64),
+                                   (2049, 1280, 128), (1100, 2304, 64)])
+def test_swiglu(pkg, oracle, m, n, k):
+    a, b = mats(oracle, m, n, k, 41)
+    b2 = oracle.synth_fp16(8, 4, n * k, std=0.02).reshape(n, k)
+    out = torch.full((m + 1, n), 0x7BFF, dtype=torch.int16, device="cuda")
+    gemm(pkg, a=dev(a), b=dev(b), b2=dev(b2), c=out, m=m, n=n, k=k, epilogue=EPI_SWIGLU)
+    g, u = matmul64(a, b), matmul64(a, b2)
+    want = g / (1.0 + np.exp(-g)) * u
+    got = host_u16(out).reshape(m + 1, n)
+    assert_close_fp16(got[:m], want, what="swiglu", abs_tol=tc_tol(want, k))
+    assert (got[m] == 0x7BFF).all()
+
+
+@pytest.mark.parametrize("m,nqh,nkvh,hd,k,batched", [(96, 8, 4, 64, 512, True), (33, 4, 2, 64, 2048, True), (100, 4, 1, 128, 64, False), (128, 12, 2, 128, 1024, False),
+                                                     (3000, 12, 2, 128, 64, False), (2500, 16, 3, 128, 64, True)])
+def test_rope_kv(pkg, oracle, m, nqh, nkvh, hd, k, batched):
+    """Rows of one sequence, and one row of each of m sequences (row_pos)."""
+    n_q, n_kv, pos0, max_pos = nqh * hd, nkvh * hd, 5, (16 if batched else m + 8)
+    n = n_q + 2 * n_kv
+    a, b = mats(oracle, m, n, k, 42)
+    pos = np.arange(m) % 13 if batched else np.arange(pos0, pos0 + m)
+    ang = pos[:, None].astype(np.float32) * np.linspace(1.0, 0.01, hd // 2, dtype=np.float32)[None]
+    cs = np.stack([np.cos(ang), np.sin(ang)], axis=-1).astype(np.float32)
+    q = torch.zeros((m, n_q), dtype=torch.int16, device="cuda")
+    rows = m * max_pos if batched else max_pos
+    kc, vc = (torch.zeros((rows, n_kv), dtype=torch.int16, device="cuda") for _ in range(2))
+    kw = dict(row_pos=torch.tensor(pos, dtype=torch.int32, device="cuda"), seq_stride=max_pos) if batched else dict(pos0=pos0)
+    gemm(pkg, a=dev(a), b=dev(b), c=q, m=m, n=n, k=k, epilogue=EPI_ROPE_KV, n_q=n_q, n_kv=n_kv, head_dim=hd, rope_cs=dev(cs), k_cache=kc,
+         v_cache=vc, max_pos=max_pos, **kw)
+    y = matmul64(a, b).astype(np.float16).astype(np.float64)
+    r = y[:, :n_q + n_kv].reshape(m, -1, hd // 2, 2)
+    c, s = cs[:, None, :, 0].astype(np.float64), cs[:, None, :, 1].astype(np.float64)
+    want = np.stack([c * r[..., 0] - s * r[..., 1], s * r[..., 0] + c * r[..., 1]], axis=-1).reshape(m, -1)
+    tol = np.repeat(np.abs(r).sum(axis=-1).reshape(m, -1), 2, axis=1) * 2.0 ** -10 + tc_tol(y, k)
+    tol += np.abs(want) * 2.0 ** -10  # one FP16 step of either input of a pair, and the result's own rounding
+    at = (np.arange(m) * max_pos + pos) if batched else pos
+    kg, vg = host_u16(kc).reshape(rows, n_kv), host_u16(vc).reshape(rows, n_kv)
+    assert_close_fp16(host_u16(q).reshape(m, n_q), want[:, :n_q], what="q", max_frac=0.1, abs_tol=tol[:, :n_q])
+    assert_close_fp16(kg[at], want[:, n_q:], what="k", max_frac=0.1, abs_tol=tol[:, n_q:])
+    assert_close_fp16(vg[at], y[:, n_q + n_kv:], what="v", abs_tol=tc_tol(y, k))
+    rest = np.setdiff1d(np.arange(rows), at)
+    assert not kg[rest].any() and not vg[rest].any()
