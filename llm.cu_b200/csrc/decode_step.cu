@@ -35,6 +35,7 @@
 #include <cstdlib>
 
 #include "gemv_common.cuh"
+#include "mma_common.cuh"
 #include "tp_common.cuh"
 
 namespace llmb {
@@ -49,7 +50,9 @@ constexpr int kDsGThreads = kDsGWarps * 32;       // 256
 constexpr int kDsSlots = 6;
 constexpr uint32_t kDsSlotBytes = 32 * 1024;
 constexpr int kDsJ = 8;                           // 16-byte chunks of x per thread: k <= 16384
-constexpr int kDsTile = 32;                       // cache rows per attention tile
+constexpr uint32_t kDsAttBytes = 16 * 1024;       // attention: partial outputs of the warps on their way to one another
+constexpr int kDsAttRows = 16;                    // cache rows per warp and attention tile
+constexpr int kDsSplitUnit = 32;                  // rows per attention split: a multiple of this
 constexpr uint32_t kPollLimit = 1u << 22;
 constexpr uint32_t kTagPollLimit = 1u << 20;  // default spins of a tagged wait: on the order of a second
 
@@ -174,11 +177,6 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
     return t;
 }
 
-__device__ __forceinline__ void cp_async16_ds(void *smem_dst, const void *gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all_ds() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 struct DsShared {
     uint64_t full_bar[kDsSlots];   // stage data has landed (bulk-copy byte count)
     uint64_t done_bar[kDsSlots];   // the 8 consumer warps of the stage have left their partials
@@ -188,10 +186,8 @@ struct DsShared {
     int fin_best_idx;
     float norm_buf[kDsGroups][512];
     float2 rope_cs[64];
-    float q_s[8 * 128];
-    float p_s[8 * kDsTile];
-    float scale_s[8];
-    float m_s[8], l_s[8];
+    uint4 q_s[8 * 128 / 8];          // attention: the eight (G real) query heads of the task's KV head, FP16
+    float att_m[kDsWarps][8], att_l[kDsWarps][8];  // per warp and head: maximum, weighted sum
     float norm_rms[kDsGroups];
     int abort_flag;
     int is_last;
@@ -272,15 +268,287 @@ __device__ __forceinline__ float stage_dot(const unsigned char *base, size_t row
     return warp_reduce_multi<NR>(acc, lane);
 }
 
+// ---- attention phase: a warp takes tiles of 16 cache rows of one KV head straight from L2 into MMA fragments ----
+// Bound: latency (a layer's cached rows are 0.3-17 MB over 148 SMs, between two grid barriers).  So there is no shared-
+// memory tile and no CTA barrier per tile: the rows are the 16 rows of mma.m16n8k16, the query heads its 8 columns, as in
+// attn_decode.cu, and every 16 bytes a lane loads are operand fragments as they lie, because the order of the contracted
+// index is free (K: lane = row group x chunk, the same chunks of q on the other side) and so is that of the output
+// dimensions (V: lane = two row pairs x chunk; elements e and e + 4 of the chunks are one 16-dimension tile).  The rows are
+// brought to L2 before the grid barrier; the warps of a CTA meet once per task.
+// Registers decide the form: the kernel has 96 per thread, the ring leaves L1 28 KB, and what the attention spills is
+// spilled in the projections as well (forms that held a whole K tile, or K across the barrier: 0.5-2 KB of spills and
+// 0.65 ms more per step, whatever they gained here).  So K comes in two halves, and at head_dim 128 two warps take the same
+// rows, each for 64 of V's dimensions.
+// 32-row tiles in shared memory with five CTA barriers each: 4.36 ms a step behind 4096 rows (8B shape); this form 3.24.
+template <int HD>
+struct WarpAttn {
+    static constexpr int KJ = HD / 32;        // chunks of 8 dimensions per lane and K row
+    static constexpr int NC = HD / 64;        // warps per 16 rows
+    static constexpr int SLOTS = kDsWarps / NC;
+
+    // V rows r, r + 1, r + 8, r + 9 of the chunk at vb
+    static __device__ __forceinline__ void load_v(uint4 (&v)[4], const __half *vb, int stride, int r, int lim) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = r + (i & 1) + 8 * (i >> 1);
+            v[i] = row < lim ? __ldcg(reinterpret_cast<const uint4 *>(vb + (size_t)row * stride)) : make_uint4(0, 0, 0, 0);
+        }
+    }
+    static __device__ __forceinline__ uint32_t word(const uint4 &v, int w) { return w == 0 ? v.x : w == 1 ? v.y : w == 2 ? v.z : v.w; }
+    // (element e of chunk a, element e of chunk b)
+    static __device__ __forceinline__ uint32_t pair(const uint4 &a, const uint4 &b, int e) {
+        return __byte_perm(word(a, e >> 1), word(b, e >> 1), (e & 1) ? 0x7632 : 0x5410);
+    }
+};
+
+// The attention phase of one layer for this CTA's tasks (task = split of a KV head's cache rows).  `wait` = the grid
+// barrier after the QKV phase.
+template <int HD, typename Wait>
+__device__ __forceinline__ void attention_phase(const DsParams &p, const DsLayer &L, DsShared &sh, unsigned char *area, int pos, int warp, int lane,
+                                                const Wait &wait, const bool &ok) {
+    using W = WarpAttn<HD>;
+    const int tid = warp * 32 + lane, gr = lane >> 2, gc = lane & 3, slot = warp / W::NC, vc = warp % W::NC;
+    const int G = p.nq / p.nkv, n_kv = p.nkv * HD, n_out = G * HD;
+    const int len_total = pos + 1, n_tasks = p.nkv * p.n_splits;
+    const float sqrt_hd = sqrtf((float)HD), rsqrt_hd = __fdiv_rn(1.0f, sqrt_hd);
+
+    int task = blockIdx.x;
+    if (task < n_tasks) {  // rows below `pos`, which earlier steps wrote, on their way to L2 before the barrier
+        const int kvh = task / p.n_splits, begin = (task % p.n_splits) * p.split_len, lim = min(begin + p.split_len, pos);
+        for (int i = tid; i < (lim - begin) * 2 * W::NC; i += kDsConsumers) {
+            const int part = i % (2 * W::NC);
+            const __half *base = part < W::NC ? L.k_cache : L.v_cache;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(base + (size_t)(begin + i / (2 * W::NC)) * n_kv + (size_t)kvh * HD + (part % W::NC) * 64));
+        }
+    }
+    wait();
+    for (; task < n_tasks && ok; task += gridDim.x) {
+        const int kvh = task / p.n_splits, split = task % p.n_splits;
+        const int begin = split * p.split_len, end = min(begin + p.split_len, len_total);
+        const __half *kb = L.k_cache + (size_t)kvh * HD, *vb = L.v_cache + (size_t)kvh * HD + vc * 64;
+        if (task != (int)blockIdx.x) named_bar_sync(1, kDsConsumers);  // the previous task is done with shared memory
+        if (tid < HD) sh.q_s[tid] = tid < G * (HD / 8) ? __ldcg(reinterpret_cast<const uint4 *>(p.q + (size_t)kvh * n_out) + tid) : make_uint4(0, 0, 0, 0);
+        int t0 = begin + slot * kDsAttRows;
+        named_bar_sync(1, kDsConsumers);
+        // of heads 2 gc and 2 gc + 1, over this warp's rows (l: this lane's share); o[e]: dimensions 8 gr + e and 8 gr + 4 + e
+        // of the warp's 64 x these heads
+        float o[4][4], m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e][0] = o[e][1] = o[e][2] = o[e][3] = 0.0f;
+        const bool real0 = 2 * gc < G, real1 = 2 * gc + 1 < G;
+        auto tile = [&]() {  // rows t0 .. t0 + 15
+            float sc[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // (row gr, heads 2 gc, + 1), (row gr + 8, same heads)
+            const uint4 *pk = reinterpret_cast<const uint4 *>(kb + (size_t)(t0 + gr) * n_kv) + gc;
+            const bool in_a = t0 + gr < end, in_b = t0 + gr + 8 < end;
+#pragma unroll 1
+            for (int j = 0; j < W::KJ; j += 2) {
+                uint4 k[4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    k[2 * i] = in_a ? __ldcg(pk + 4 * (j + i)) : make_uint4(0, 0, 0, 0);
+                    k[2 * i + 1] = in_b ? __ldcg(pk + n_kv + 4 * (j + i)) : make_uint4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint4 q = sh.q_s[gr * (HD / 8) + gc + 4 * (j + i)];
+                    const uint32_t a0[4] = {k[2 * i].x, k[2 * i + 1].x, k[2 * i].y, k[2 * i + 1].y};
+                    mma_16816(sc, a0, q.x, q.y);
+                    const uint32_t a1[4] = {k[2 * i].z, k[2 * i + 1].z, k[2 * i].w, k[2 * i + 1].w};
+                    mma_16816(sc, a1, q.z, q.w);
+                }
+            }
+            uint4 v[4];  // rows 2 gc, 2 gc + 1, 2 gc + 8, 2 gc + 9, chunk gr
+            W::load_v(v, vb + gr * 8, n_kv, t0 + 2 * gc, end);
+            // columns past G hold exact zeros: not divided (an IEEE division of zero leaves the fast path)
+            sc[0] = real0 ? (in_a ? div_by_const(sc[0], sqrt_hd, rsqrt_hd) : -INFINITY) : 0.0f;
+            sc[1] = real1 ? (in_a ? div_by_const(sc[1], sqrt_hd, rsqrt_hd) : -INFINITY) : 0.0f;
+            sc[2] = real0 ? (in_b ? div_by_const(sc[2], sqrt_hd, rsqrt_hd) : -INFINITY) : 0.0f;
+            sc[3] = real1 ? (in_b ? div_by_const(sc[3], sqrt_hd, rsqrt_hd) : -INFINITY) : 0.0f;
+            float t_0 = fmaxf(sc[0], sc[2]), t_1 = fmaxf(sc[1], sc[3]);
+#pragma unroll
+            for (int x = 4; x < 32; x <<= 1) {
+                t_0 = fmaxf(t_0, __shfl_xor_sync(0xffffffffu, t_0, x));
+                t_1 = fmaxf(t_1, __shfl_xor_sync(0xffffffffu, t_1, x));
+            }
+            const float n0 = fmaxf(m0, t_0), n1 = fmaxf(m1, t_1);  // finite: row t0 is inside
+            const float s0 = expf(m0 - n0), s1 = expf(m1 - n1);    // 0 on the first tile
+            m0 = n0;
+            m1 = n1;
+            float p0 = expf(sc[0] - n0), p1 = expf(sc[1] - n1), p2 = expf(sc[2] - n0), p3 = expf(sc[3] - n1);
+            l0 = l0 * s0 + (p0 + p2);
+            l1 = l1 * s1 + (p1 + p3);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                o[e][0] *= s0;
+                o[e][1] *= s1;
+                o[e][2] *= s0;
+                o[e][3] *= s1;
+            }
+            // probabilities as three FP16 terms (11 bits each: the FP32 value, to 2^-25 absolute where p < 1), transposed into
+            // operand layout
+            uint32_t pt[3][2];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const __half2 h01 = __floats2half2_rn(p0, p1), h23 = __floats2half2_rn(p2, p3);
+                const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
+                pt[i][0] = movmatrix_trans(*reinterpret_cast<const uint32_t *>(&h01));
+                pt[i][1] = movmatrix_trans(*reinterpret_cast<const uint32_t *>(&h23));
+                p0 -= f01.x; p1 -= f01.y; p2 -= f23.x; p3 -= f23.y;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const uint32_t a[4] = {W::pair(v[0], v[1], e), W::pair(v[0], v[1], e + 4), W::pair(v[2], v[3], e), W::pair(v[2], v[3], e + 4)};
+#pragma unroll
+                for (int i = 0; i < 3; ++i) mma_16816(o[e], a, pt[i][0], pt[i][1]);
+            }
+        };
+#pragma unroll 1
+        for (; t0 < end; t0 += W::SLOTS * kDsAttRows) tile();
+        // ---- the warps meet: common maximum per head; outputs as register images, those of `entries` slots at a time ----
+#pragma unroll
+        for (int x = 4; x < 32; x <<= 1) {
+            l0 += __shfl_xor_sync(0xffffffffu, l0, x);
+            l1 += __shfl_xor_sync(0xffffffffu, l1, x);
+        }
+        if (gr == 0) *reinterpret_cast<float2 *>(&sh.att_m[warp][2 * gc]) = make_float2(m0, m1);
+        named_bar_sync(1, kDsConsumers);
+        const int active = min(W::SLOTS, max(0, (end - begin + kDsAttRows - 1) / kDsAttRows));  // slots with rows
+        float M0 = -INFINITY, M1 = -INFINITY;
+#pragma unroll 4
+        for (int w = 0; w < active; ++w) {
+            const float2 t = *reinterpret_cast<const float2 *>(&sh.att_m[w * W::NC + vc][2 * gc]);
+            M0 = fmaxf(M0, t.x);
+            M1 = fmaxf(M1, t.y);
+        }
+        const float f0 = slot < active ? expf(m0 - M0) : 0.0f, f1 = slot < active ? expf(m1 - M1) : 0.0f;
+        if (gr == 0) *reinterpret_cast<float2 *>(&sh.att_l[warp][2 * gc]) = make_float2(l0 * f0, l1 * f1);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            o[e][0] *= f0;
+            o[e][1] *= f1;
+            o[e][2] *= f0;
+            o[e][3] *= f1;
+        }
+        const int lanes = G <= 4 ? 16 : 32, image = 16 * lanes;  // lanes with real heads
+        const int entries = min(W::SLOTS, (int)(kDsAttBytes / 4) / (image * W::NC));
+        const bool holds = G > 4 || gc < 2;
+        float *img = reinterpret_cast<float *>(area), *own = img + (G <= 4 ? gr * 2 + gc : lane);
+        for (int base = entries; base < active; base += entries) {  // the slots past the entries hand theirs down
+            if (base > entries) named_bar_sync(1, kDsConsumers);
+            if (slot >= base && slot < base + entries && holds) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) own[((slot - base) * W::NC + vc) * image + i * lanes] = o[i >> 2][i & 3];
+            }
+            named_bar_sync(1, kDsConsumers);
+            if (slot < entries && base + slot < active && holds) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) o[i >> 2][i & 3] += own[warp * image + i * lanes];
+            }
+        }
+        if (slot < entries && holds) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) own[warp * image + i * lanes] = o[i >> 2][i & 3];
+        }
+        named_bar_sync(1, kDsConsumers);
+        const size_t pbase = ((size_t)kvh * p.n_splits + split) * G;
+        for (int r = tid; r < image * W::NC; r += kDsConsumers) {
+            float num = 0.0f;
+#pragma unroll 4
+            for (int w = 0; w < min(active, entries); ++w) num += img[w * W::NC * image + r];
+            const int i = (r % image) / lanes, at = r % lanes;
+            const int head = 2 * (G <= 4 ? at & 1 : at & 3) + (i & 1), gg = G <= 4 ? at >> 1 : at >> 2;
+            const int dim = r / image * 64 + 8 * gg + ((i >> 1) & 1) * 4 + (i >> 2);
+            if (head >= G) continue;
+            if (p.n_splits == 1) {
+                float den = 0.0f;
+#pragma unroll 4
+                for (int w = 0; w < active; ++w) den += sh.att_l[w * W::NC][head];
+                p.attn[(size_t)kvh * n_out + head * HD + dim] = __float2half_rn(__fdiv_rn(num, den));
+            } else {
+                p.part_o[(pbase + head) * HD + dim] = num;
+            }
+        }
+        if (p.n_splits == 1) continue;
+        if (tid < G) {
+            float mm = -INFINITY, ll = 0.0f;
+            for (int w = 0; w < active; ++w) {
+                mm = fmaxf(mm, sh.att_m[w * W::NC][tid]);
+                ll += sh.att_l[w * W::NC][tid];
+            }
+            p.part_ml[(pbase + tid) * 2] = mm;
+            p.part_ml[(pbase + tid) * 2 + 1] = ll;
+        }
+        named_bar_sync(1, kDsConsumers);
+        if (tid == 0) {
+            __threadfence();  // cumulative: orders the whole CTA's partials before the count
+            const int prev = atomicAdd(&p.attn_counters[kvh], 1);
+            sh.is_last = (prev == p.n_splits - 1);
+            if (sh.is_last) p.attn_counters[kvh] = 0;
+        }
+        named_bar_sync(1, kDsConsumers);
+        if (sh.is_last) {
+            __threadfence();
+            // Merge in split order.  All loads of a step are independent, so each step costs
+            // about one L2 round trip: (1) every (split, head) max and sum, (2) the weights,
+            // (3) the partial outputs in batches of eight splits.
+            const int n_used = min(p.n_splits, (len_total + p.split_len - 1) / p.split_len);
+            const size_t gbase = (size_t)kvh * p.n_splits * G;
+            float *m_all = sh.norm_buf[0];  // idle during attention: [split][head]
+            float *l_all = sh.norm_buf[1];
+            for (int e = tid; e < n_used * G; e += kDsConsumers) {
+                const float2 ml = __ldcg(reinterpret_cast<const float2 *>(&p.part_ml[(gbase + e) * 2]));
+                m_all[e] = ml.x;
+                l_all[e] = ml.y;
+            }
+            named_bar_sync(1, kDsConsumers);
+            float wgt_keep = 0.0f;
+            int e_keep = -1;
+            if (tid < n_used * G && tid < 512) {
+                const int hh = tid % G;
+                float M = -INFINITY;
+                for (int sidx = 0; sidx < n_used; ++sidx) M = fmaxf(M, m_all[sidx * G + hh]);
+                const float m = m_all[tid];
+                wgt_keep = (m == -INFINITY) ? 0.0f : expf(m - M);
+                e_keep = tid;
+            }
+            named_bar_sync(1, kDsConsumers);
+            if (e_keep >= 0) m_all[e_keep] = wgt_keep;  // m_all now holds the weights
+            named_bar_sync(1, kDsConsumers);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int o = tid + kDsConsumers * i;
+                if (o < n_out) {
+                    const int hh = o / HD, dd = o % HD;
+                    float num = 0.0f, den = 0.0f;
+                    for (int s0 = 0; s0 < n_used; s0 += 8) {
+                        float v[8];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u)
+                            v[u] = (s0 + u < n_used) ? __ldcg(&p.part_o[(gbase + (size_t)(s0 + u) * G + hh) * HD + dd]) : 0.0f;
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            if (s0 + u < n_used) {
+                                const float wgt = m_all[(s0 + u) * G + hh];
+                                num = fmaf(wgt, v[u], num);
+                                den = fmaf(wgt, l_all[(s0 + u) * G + hh], den);
+                            }
+                        }
+                    }
+                    p.attn[(size_t)kvh * n_out + o] = __float2half_rn(__fdiv_rn(num, den));
+                }
+            }
+        }
+    }
+}
+
 // kTp = false compiles every tensor-parallel branch out of the single-GPU kernel.
 template <bool kTp>
 __global__ void __launch_bounds__(kDsThreads, 1) decode_step_kernel(const DsParams p) {
     extern __shared__ __align__(128) unsigned char ds_smem[];
     unsigned char *ring = ds_smem;
-    __half *k_tile = reinterpret_cast<__half *>(ds_smem + (size_t)kDsSlots * kDsSlotBytes);
-    __half *v_tile = k_tile + kDsTile * 128;
+    unsigned char *att_area = ds_smem + (size_t)kDsSlots * kDsSlotBytes;
     // the per-layer pointer table, copied once: phase switches must not wait on global memory
-    DsLayer *layer_s = reinterpret_cast<DsLayer *>(v_tile + kDsTile * 128);
+    DsLayer *layer_s = reinterpret_cast<DsLayer *>(att_area + kDsAttBytes);
     __shared__ DsShared sh;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -513,7 +781,6 @@ __global__ void __launch_bounds__(kDsThreads, 1) decode_step_kernel(const DsPara
     if (p.hidden && blockIdx.x == 0)
         for (int i = tid; i < p.d; i += kDsConsumers) p.hidden[i] = emb[i];
 
-    const int G = p.nq / p.nkv;
     // profiling aid: thread 0 of every CTA stamps the global timer four times per phase
     const int trace_row = (p.trace && tid == 0) ? (int)blockIdx.x : -1;
     auto stamp = [&](int phase, int which) {
@@ -616,7 +883,7 @@ __global__ void __launch_bounds__(kDsThreads, 1) decode_step_kernel(const DsPara
             // attention tiles, idle in this phase).  148 x 512 threads polling the row took enough of L2's bandwidth
             // to slow every round of polls: asking for two chunks at once instead of one cost 5 % of the step, and
             // leaving the polls to one group gained 4 % (430 -> 446 tok/s at two GPUs); a pause between rounds, nothing.
-            uint4 *x_s = reinterpret_cast<uint4 *>(k_tile);  // d_model <= 8192 halves = 16 KB = the K and V tile
+            uint4 *x_s = reinterpret_cast<uint4 *>(att_area);  // d_model <= 8192 halves = 16 KB = the attention's area
 #pragma unroll
             for (int j = 0; j < kDsJ / 2; ++j) {
                 xh[j] = make_uint4(0, 0, 0, 0);
@@ -738,174 +1005,12 @@ __global__ void __launch_bounds__(kDsThreads, 1) decode_step_kernel(const DsPara
             const int l = ph >> 2;
             // ------------------------------ attention ------------------------------
             stamp(tphase, 0);
-            const DsLayer &L = layer_s[l];
-            const int HD = p.hd;
-            const int chunks = HD >> 3;
-            const int len_total = pos + 1;
-            const int n_tasks = p.nkv * p.n_splits;
-            const float inv_den = sqrtf((float)HD);
-            int tpd = kDsConsumers / (kDsTile * G);  // threads per (row, head) dot product
-            tpd = tpd < 1 ? 1 : (tpd > 4 ? 4 : tpd);
-            const int n_out = G * HD;
-            auto load_rows = [&](int kvh, int t0, int r_begin, int r_end) {
-                for (int c = tid + r_begin * chunks; c < r_end * chunks; c += kDsConsumers) {
-                    const int r = c / chunks, ch = c % chunks;
-                    const size_t goff = (size_t)(t0 + r) * n_kv + (size_t)kvh * HD + ch * 8;
-                    cp_async16_ds(&k_tile[r * HD + ((ch ^ (r & 7)) * 8)], L.k_cache + goff);
-                    cp_async16_ds(&v_tile[r * HD + ch * 8], L.v_cache + goff);
-                }
+            auto wait = [&]() {
+                grid_wait();
+                stamp(tphase, 1);
             };
-            // Cache rows below `pos` were written by earlier steps: the first tile of this CTA's first
-            // task is requested before waiting for the other CTAs' q/k/v rows of this step.
-            int pre_rows = 0;
-            if ((int)blockIdx.x < n_tasks) {
-                const int kvh = blockIdx.x / p.n_splits, begin = (blockIdx.x % p.n_splits) * p.split_len;
-                pre_rows = max(0, min(kDsTile, min(begin + p.split_len, pos) - begin));
-                load_rows(kvh, begin, 0, pre_rows);
-            }
-            grid_wait();
-            stamp(tphase, 1);
-            for (int task = blockIdx.x; task < n_tasks && ok; task += gridDim.x) {
-                const int kvh = task / p.n_splits, split = task % p.n_splits;
-                const int begin = split * p.split_len;
-                const int end = min(begin + p.split_len, len_total);
-                if (task != (int)blockIdx.x) named_bar_sync(1, kDsConsumers);  // previous task is done with shared memory
-                for (int i = tid; i < n_out; i += kDsConsumers) sh.q_s[i] = __half2float(__ldcg(&p.q[(size_t)kvh * n_out + i]));
-                if (tid < G) { sh.m_s[tid] = -INFINITY; sh.l_s[tid] = 0.0f; }
-                float acc[2] = {0.0f, 0.0f};
-                for (int t0 = begin; t0 < end; t0 += kDsTile) {
-                    const int rows = min(kDsTile, end - t0);
-                    const bool first = task == (int)blockIdx.x && t0 == begin;
-                    if (!first) named_bar_sync(1, kDsConsumers);  // previous tile consumed
-                    load_rows(kvh, t0, first ? pre_rows : 0, rows);
-                    cp_async_wait_all_ds();
-                    named_bar_sync(1, kDsConsumers);
-                    // scores: dot = head * tile + row, split over tpd adjacent lanes
-                    {
-                        const int dot = tid / tpd, part = tid % tpd;
-                        const int hh = dot / kDsTile, r = dot % kDsTile;
-                        float sacc = 0.0f;
-                        if (hh < G && r < rows) {
-                            const int cpp = chunks / tpd;
-                            for (int cc = 0; cc < cpp; ++cc) {
-                                const int ch = part * cpp + cc;
-                                const uint4 kv = *reinterpret_cast<const uint4 *>(&k_tile[r * HD + ((ch ^ (r & 7)) * 8)]);
-                                const __half2 *kh = reinterpret_cast<const __half2 *>(&kv);
-                                const float *qp = &sh.q_s[hh * HD + ch * 8];
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    const float2 f = __half22float2(kh[e]);
-                                    sacc = fmaf(qp[2 * e], f.x, sacc);
-                                    sacc = fmaf(qp[2 * e + 1], f.y, sacc);
-                                }
-                            }
-                        }
-                        for (int m = tpd >> 1; m >= 1; m >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, m);
-                        if (hh < G && part == 0) sh.p_s[hh * kDsTile + r] = (r < rows) ? __fdiv_rn(sacc, inv_den) : -INFINITY;
-                    }
-                    named_bar_sync(1, kDsConsumers);
-                    if (warp < G) {  // online softmax bookkeeping of head `warp` (one tile row per lane)
-                        static_assert(kDsTile == 32, "one score per lane");
-                        const float s0 = sh.p_s[warp * kDsTile + lane];
-                        const float tmax = warp_max(s0);
-                        const float m_old = sh.m_s[warp];
-                        const float m_new = fmaxf(m_old, tmax);
-                        const float sc = (m_old == -INFINITY) ? 0.0f : expf(m_old - m_new);
-                        const float e0 = (lane < rows) ? expf(s0 - m_new) : 0.0f;
-                        sh.p_s[warp * kDsTile + lane] = e0;
-                        const float ssum = warp_sum(e0);
-                        __syncwarp();
-                        if (lane == 0) {
-                            sh.scale_s[warp] = sc;
-                            sh.m_s[warp] = m_new;
-                            sh.l_s[warp] = sh.l_s[warp] * sc + ssum;
-                        }
-                    }
-                    named_bar_sync(1, kDsConsumers);
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const int o = tid + kDsConsumers * i;
-                        if (o < n_out) {
-                            const int hh = o / HD, dd = o % HD;
-                            float a = acc[i] * sh.scale_s[hh];
-                            const float *pp = &sh.p_s[hh * kDsTile];
-                            for (int r = 0; r < rows; ++r) a = fmaf(pp[r], __half2float(v_tile[r * HD + dd]), a);
-                            acc[i] = a;
-                        }
-                    }
-                }
-                named_bar_sync(1, kDsConsumers);
-                const size_t pbase = ((size_t)kvh * p.n_splits + split) * G;
-                if (tid < G) {
-                    p.part_ml[(pbase + tid) * 2] = sh.m_s[tid];
-                    p.part_ml[(pbase + tid) * 2 + 1] = sh.l_s[tid];
-                }
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int o = tid + kDsConsumers * i;
-                    if (o < n_out) p.part_o[(pbase + o / HD) * HD + (o % HD)] = acc[i];
-                }
-                named_bar_sync(1, kDsConsumers);
-                if (tid == 0) {
-                    __threadfence();  // cumulative: orders the whole CTA's partials before the count
-                    const int prev = atomicAdd(&p.attn_counters[kvh], 1);
-                    sh.is_last = (prev == p.n_splits - 1);
-                    if (sh.is_last) p.attn_counters[kvh] = 0;
-                }
-                named_bar_sync(1, kDsConsumers);
-                if (sh.is_last) {
-                    __threadfence();
-                    // Merge in split order.  All loads of a step are independent, so each step costs
-                    // about one L2 round trip: (1) every (split, head) max and sum, (2) the weights,
-                    // (3) the partial outputs in batches of eight splits.
-                    const int n_used = min(p.n_splits, (len_total + p.split_len - 1) / p.split_len);
-                    const size_t gbase = (size_t)kvh * p.n_splits * G;
-                    float *m_all = sh.norm_buf[0];  // idle during attention: [split][head]
-                    float *l_all = sh.norm_buf[1];
-                    for (int e = tid; e < n_used * G; e += kDsConsumers) {
-                        const float2 ml = __ldcg(reinterpret_cast<const float2 *>(&p.part_ml[(gbase + e) * 2]));
-                        m_all[e] = ml.x;
-                        l_all[e] = ml.y;
-                    }
-                    named_bar_sync(1, kDsConsumers);
-                    float wgt_keep = 0.0f;
-                    int e_keep = -1;
-                    if (tid < n_used * G && tid < 512) {
-                        const int hh = tid % G;
-                        float M = -INFINITY;
-                        for (int sidx = 0; sidx < n_used; ++sidx) M = fmaxf(M, m_all[sidx * G + hh]);
-                        const float m = m_all[tid];
-                        wgt_keep = (m == -INFINITY) ? 0.0f : expf(m - M);
-                        e_keep = tid;
-                    }
-                    named_bar_sync(1, kDsConsumers);
-                    if (e_keep >= 0) m_all[e_keep] = wgt_keep;  // m_all now holds the weights
-                    named_bar_sync(1, kDsConsumers);
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const int o = tid + kDsConsumers * i;
-                        if (o < n_out) {
-                            const int hh = o / HD, dd = o % HD;
-                            float num = 0.0f, den = 0.0f;
-                            for (int s0 = 0; s0 < n_used; s0 += 8) {
-                                float v[8];
-#pragma unroll
-                                for (int u = 0; u < 8; ++u)
-                                    v[u] = (s0 + u < n_used) ? __ldcg(&p.part_o[(gbase + (size_t)(s0 + u) * G + hh) * HD + dd]) : 0.0f;
-#pragma unroll
-                                for (int u = 0; u < 8; ++u) {
-                                    if (s0 + u < n_used) {
-                                        const float wgt = m_all[(s0 + u) * G + hh];
-                                        num = fmaf(wgt, v[u], num);
-                                        den = fmaf(wgt, l_all[(s0 + u) * G + hh], den);
-                                    }
-                                }
-                            }
-                            p.attn[(size_t)kvh * n_out + o] = __float2half_rn(__fdiv_rn(num, den));
-                        }
-                    }
-                }
-            }
+            if (p.hd == 128) attention_phase<128>(p, layer_s[l], sh, att_area, pos, warp, lane, wait, ok);
+            else attention_phase<64>(p, layer_s[l], sh, att_area, pos, warp, lane, wait, ok);
             stamp(tphase, 2);
             grid_arrive();
             stamp(tphase, 3);
@@ -1037,7 +1142,7 @@ extern "C" int llmb_decode_step(const LlmbDecodeStepArgs *a, llmb_stream_t strea
         return LLMB_ERR_INVALID;
     if (a->with_logits && (!a->lm_head || !a->g_final || !a->logits || !a->next_token)) return LLMB_ERR_INVALID;
     if (a->n_layers <= 0 || a->n_kv_heads <= 0 || a->n_q_heads % a->n_kv_heads || a->n_splits <= 0 ||
-        a->split_len <= 0 || (a->split_len % kDsTile) != 0 || a->n_splits > a->max_splits)
+        a->split_len <= 0 || (a->split_len % kDsSplitUnit) != 0 || a->n_splits > a->max_splits)
         return LLMB_ERR_INVALID;
     const int G = a->n_q_heads / a->n_kv_heads;
     if (a->n_splits * G > 512) return LLMB_ERR_INVALID;  // the merge keeps one weight per (split, head) in shared memory
@@ -1113,7 +1218,7 @@ extern "C" int llmb_decode_step(const LlmbDecodeStepArgs *a, llmb_stream_t strea
         p.x_alt = reinterpret_cast<__half *>(a->x_alt);
     }
 
-    const size_t smem = (size_t)kDsSlots * kDsSlotBytes + (size_t)2 * kDsTile * 128 * sizeof(__half) +
+    const size_t smem = (size_t)kDsSlots * kDsSlotBytes + kDsAttBytes +
                         (size_t)a->n_layers * sizeof(DsLayer);
     static size_t smem_limit[kMaxDevices] = {}, set_plain[kMaxDevices] = {}, set_tp[kMaxDevices] = {};  // per device
     const int slot = current_device_slot();

@@ -223,14 +223,15 @@ int kernels_per_step(const Engine *e, bool with_logits) {
     return 1 + 5 * e->layers + (with_logits ? 2 : 1);
 }
 
-// The whole step as one persistent kernel.  Attention splits: 32-row tiles, doubled until the
-// task count fits about two waves of CTAs.
+// The whole step as one persistent kernel.  Attention splits of a KV head: as many as there are CTAs per KV head, of at
+// least 128 rows (one round of a CTA's warps at head_dim 128).  Splits of 32 to 256 rows behind 128 cached rows differ by
+// less than two runs of the same one (198.2 to 203.4 ms for a prompt of 128 tokens and 63 steps), and so do minima of 64
+// and 128 behind 4096; with 128 the summation order picks the reference's token on every step of the full-depth fixture.
 int launch_step_kernel(Engine *e, bool with_logits, int len) {
     const Llama3Config &c = e->model->config;
-    int split_len = 32;
     const int G = e->nq / e->nkv;
-    while (e->nkv * ((len + split_len - 1) / split_len) > 2 * e->sm_count || ((len + split_len - 1) / split_len) * G > 512)
-        split_len *= 2;
+    const int most = std::max(1, std::min({e->sm_count / e->nkv, 512 / G, 32, e->step_max_splits}));
+    const int split_len = std::max(128, ((len + most - 1) / most + 31) / 32 * 32);
     LlmbDecodeStepArgs a = {};
     a.layers = e->d_layers;
     a.n_layers = e->layers;
