@@ -27,6 +27,8 @@
 //   warps     0 = TMA producer, 1 = MMA issuer (one lane) + tensor-memory owner, 2-5 = epilogue; thread =
 //             tensor-memory lane = one weight row n, holding the values of all activation rows for it.
 // Every mbarrier wait is bounded (status word, see llmb_device_status).
+#include <type_traits>
+
 #include "gemm_common.cuh"
 #include "tp_common.cuh"
 
@@ -49,23 +51,16 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
-// The S slices' partial sums of one element, added in slice order (`last_first`: from the last slice to the first).
-// rbase[z] + off = its address in slice z's block of partial sums as seen from this CTA.
-__device__ __forceinline__ float gather_slices(const uint32_t (&rbase)[8], int n_slices, uint32_t off, bool last_first) {
-    float t[8];
+// The sum of S slices' partial sums in slice order (`last_first`: from the last slice to the first).
+template <int S>
+__device__ __forceinline__ float add_slices(const float (&t)[S], bool last_first) {
+    float up = 0.0f, down = 0.0f;
 #pragma unroll
-    for (int z = 0; z < 8; ++z) {
-        t[z] = 0.0f;
-        if (z < n_slices) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(t[z]) : "r"(rbase[z] + off) : "memory");
+    for (int z = 0; z < S; ++z) {
+        up += t[z];
+        down += t[S - 1 - z];
     }
-    float sum = 0.0f;
-#pragma unroll
-    for (int z = 0; z < 8; ++z)
-        if (z < n_slices && !last_first) sum += t[z];
-#pragma unroll
-    for (int z = 7; z >= 0; --z)
-        if (z < n_slices && last_first) sum += t[z];
-    return sum;
+    return last_first ? down : up;
 }
 
 template <bool DUAL>
@@ -197,10 +192,11 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             umma_commit(&acc_bar);  // arrives even after a failed wait, so the epilogue never waits forever
         }
     }
-    // ---- epilogue: thread = weight row n0 + lane_group + lane.  The accumulators go to shared memory first (over
-    // the ring), [accumulator][activation row b][weight row]; the rows are then finished four at a time in a loop
-    // that is NOT unrolled over all rows: a CTA runs its epilogue once, so every instruction of it is fetched
-    // cold, and the fully unrolled form (five epilogues x 32 rows) cost 5-19 us of instruction fetch per launch.
+    // ---- epilogue: thread = weight row n0 + lane_group + lane.  Loops over four or eight rows that are NOT unrolled over
+    // all of them: a CTA runs its epilogue once, so every instruction of it is fetched cold, and the fully unrolled form
+    // (five epilogues x 32 rows) cost 5-19 us of instruction fetch per launch.  With a test per possible slice and
+    // everything through shared memory it took 14 / 11 / 37 / 10 us of the four projections of a layer at 96 rows (last
+    // accumulator to last store); this form 14 / 10 / 10 / 8.
     const int lane_group = (warp & 3) * 32;
     const int nl = lane_group + lane;
     const int n = n0 + nl;
@@ -215,126 +211,129 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     // every load of the ring has landed and every MMA has read it (acc_bar): the ring is free
     const uint32_t taddr = tmem_base + ((uint32_t)lane_group << 16);
-    auto spill = [&](int b0, int red_rows, int at) {  // columns b0 .. b0 + 31 to rows at .. of the block of partial sums
-        uint32_t v[32];
-        tmem_ld32(taddr + b0, v);
-#pragma unroll
-        for (int b = 0; b < 32; ++b) red_own[(at + b) * kBM + nl] = v[b];
-        if (DUAL) {
-            tmem_ld32(taddr + nx + b0, v);
-#pragma unroll
-            for (int b = 0; b < 32; ++b) red_own[(red_rows + at + b) * kBM + nl] = v[b];
-        }
-    };
-    // Split K: all slices of the tile meet, then CTA r of the cluster finishes activation rows r * nx/S ..; without a split
-    // a thread only reads back what it wrote itself, 32 rows at a time, so no barrier is needed.
+    // Split K: every slice leaves its partial sums in its shared memory as [accumulator][activation row][weight row].
     if (clustered) {
         if (warp >= 2) {
 #pragma unroll 1
-            for (int b0 = 0; b0 < nx; b0 += 32) spill(b0, nx, b0);
+            for (int b0 = 0; b0 < (DUAL ? 2 : 1) * nx; b0 += 32) {
+                uint32_t v[32];
+                tmem_ld32(taddr + b0, v);
+#pragma unroll
+                for (int b = 0; b < 32; ++b) red_own[(b0 + b) * kBM + nl] = v[b];
+            }
         }
         cluster_sync_all();  // all slices of the tile are in shared memory
     }
     if (threadIdx.x == 64) stamp(6);
     if (warp >= 2) {
-        const int nb = clustered ? nx / p.splits : 32, red_rows = clustered ? nx : 32;
-        const int first = clustered ? slice * nb : 0, past = clustered ? first + nb : nx;
-#pragma unroll 1
-        for (int b_lo = first; b_lo < past; b_lo += nb) {
-            if (!clustered) spill(b_lo, 32, 0);  // warp-collective: every lane takes part
-            const int red0 = clustered ? 0 : b_lo;
-            if (ok && n < p.N) {  // the last weight tile may reach past N (its rows are zero-filled by TMA)
-                uint32_t rbase[8];
-                const uint32_t red = smem_u32(ring);
+        // Output element (b, n): the 32 lanes of a warp hold 32 consecutive n, so each store of a warp is one 64-byte run of
+        // row b.  R rows at a time: their loads first, then their stores (a load after a store to the same array would have
+        // to wait for it).
+        const bool valid = ok && n < p.N;  // the last weight tile may reach past N (its rows are zero-filled by TMA)
+        const int half_dim = p.head_dim >> 1;
+        const bool is_q = n < p.n_q, is_v = n >= p.n_q + p.n_kv;
+        const int local = is_q ? n : (is_v ? n - p.n_q - p.n_kv : n - p.n_q);
+        const int pair = half_dim > 0 ? (local >> 1) % half_dim : 0;
+        const unsigned int tag = p.epilogue == LLMB_EPI_TP_SCATTER ? __ldg(p.tp_seq) + (unsigned int)p.tp_index + 1u : 0u;
+        auto finish = [&](int b0, int b_hi, auto &val, auto &val2) {
+            constexpr int R = sizeof(val) / sizeof(float);
+            if (!DUAL && p.epilogue == LLMB_EPI_TP_SCATTER) {
+                // tensor parallel: this rank's partial sums go, tagged, to every rank's receive buffer
+                const size_t slot0 = tp_rows_slot(p.tp_size, p.N, p.tp_index, p.tp_rank, 0, n);
 #pragma unroll
-                for (int z = 0; z < 8; ++z) {
-                    rbase[z] = red;
-                    if (clustered && z < p.splits) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbase[z]) : "r"(red), "r"(z));
-                }
-                const int n_slices = clustered ? p.splits : 1;
-                const int b_hi = min(b_lo + nb, p.M);
-                // Output element (b, n): the 32 lanes of a warp hold 32 consecutive n, so each store of a warp is one
-                // 64-byte run of row b.  Loads of four rows first, then their stores.
-                const int half_dim = p.head_dim >> 1;
-                const bool is_q = n < p.n_q, is_v = n >= p.n_q + p.n_kv;
-                const int local = is_q ? n : (is_v ? n - p.n_q - p.n_kv : n - p.n_q);
-                const int pair = half_dim > 0 ? (local >> 1) % half_dim : 0;
-                const unsigned int tag = p.epilogue == LLMB_EPI_TP_SCATTER ? __ldg(p.tp_seq) + (unsigned int)p.tp_index + 1u : 0u;
-#pragma unroll 1
-                for (int b0 = b_lo; b0 < b_hi; b0 += 4) {
-                    float val[4], val2[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int b = min(b0 + i, b_hi - 1);
-                        const uint32_t off = (uint32_t)(((b - red0) * kBM + nl) * 4);
-                        val[i] = gather_slices(rbase, n_slices, off, last_first);
-                        val2[i] = DUAL ? gather_slices(rbase, n_slices, off + (uint32_t)(red_rows * kBM * 4), last_first) : 0.0f;
-                    }
-                    if (!DUAL && p.epilogue == LLMB_EPI_TP_SCATTER) {
-                        // tensor parallel: this rank's partial sums go, tagged, to every rank's receive buffer
-                        const size_t slot0 = tp_rows_slot(p.tp_size, p.N, p.tp_index, p.tp_rank, 0, n);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            if (b0 + i < b_hi) {
-                                const size_t off = slot0 + (size_t)(b0 + i) * p.N * 8;
-                                for (int r = 0; r < p.tp_size; ++r)
-                                    asm volatile("st.relaxed.sys.global.v2.b32 [%0], {%1, %2};" ::"l"(p.tp_peer[r] + off), "r"(__float_as_uint(val[i])),
-                                                 "r"(tag)
-                                                 : "memory");
-                            }
-                        }
-                    } else if (DUAL) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            if (b0 + i < b_hi) p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(silu_gemm(val[i]) * val2[i]);
-                    } else if (p.epilogue == LLMB_EPI_STORE) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            if (b0 + i < b_hi) p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(val[i]);
-                    } else if (p.epilogue == LLMB_EPI_RESIDUAL) {
-                        // the residual values of the four rows first, then the stores: a load after a store to the same
-                        // array would have to wait for it
-                        __half res[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) res[i] = __ldcg(p.c + (size_t)min(b0 + i, b_hi - 1) * p.N + n);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            if (b0 + i < b_hi)
-                                p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(__half2float(__float2half_rn(val[i])) + __half2float(res[i]));
-                    } else {  // LLMB_EPI_ROPE_KV: the pair (even n, n + 1) sits in neighbouring lanes
-                        float2 cs[4];
-                        int pos[4];
-                        size_t cache_row[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int b = min(b0 + i, b_hi - 1);
-                            cs[i] = is_v ? make_float2(1.0f, 0.0f) : __ldg(p.rope_cs + (size_t)b * half_dim + pair);
-                            pos[i] = kv_position(p, b, cache_row[i]);
-                        }
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int b = b0 + i;
-                            // b and b_hi are the same in all lanes, so the shuffle is executed by the whole warp (N is a
-                            // multiple of 32 whenever this epilogue is used: whole heads)
-                            if (b < b_hi) {
-                                const float mine = __half2float(__float2half_rn(val[i]));
-                                const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
-                                __half out;
-                                if (is_v) {
-                                    out = __float2half_rn(val[i]);
-                                } else {
-                                    out = __float2half_rn((n & 1) ? __fmaf_rn(cs[i].y, other, __fmul_rn(cs[i].x, mine))
-                                                                  : __fmaf_rn(cs[i].x, mine, -__fmul_rn(cs[i].y, other)));
-                                }
-                                if (is_q) {
-                                    p.c[(size_t)b * p.n_q + n] = out;
-                                } else {
-                                    if (pos[i] >= 0 && pos[i] < p.max_pos) (is_v ? p.v_cache : p.k_cache)[cache_row[i] * p.n_kv + local] = out;
-                                }
-                            }
-                        }
+                for (int i = 0; i < R; ++i) {
+                    if (valid && b0 + i < b_hi) {
+                        const size_t off = slot0 + (size_t)(b0 + i) * p.N * 8;
+                        for (int r = 0; r < p.tp_size; ++r)
+                            asm volatile("st.relaxed.sys.global.v2.b32 [%0], {%1, %2};" ::"l"(p.tp_peer[r] + off), "r"(__float_as_uint(val[i])),
+                                         "r"(tag)
+                                         : "memory");
                     }
                 }
+            } else if (DUAL) {
+#pragma unroll
+                for (int i = 0; i < R; ++i)
+                    if (valid && b0 + i < b_hi) p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(silu_gemm(val[i]) * val2[i]);
+            } else if (p.epilogue == LLMB_EPI_STORE) {
+#pragma unroll
+                for (int i = 0; i < R; ++i)
+                    if (valid && b0 + i < b_hi) p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(val[i]);
+            } else if (p.epilogue == LLMB_EPI_RESIDUAL) {
+                __half res[R];
+#pragma unroll
+                for (int i = 0; i < R; ++i) res[i] = valid && b0 + i < b_hi ? __ldcg(p.c + (size_t)(b0 + i) * p.N + n) : __half(0.0f);
+#pragma unroll
+                for (int i = 0; i < R; ++i)
+                    if (valid && b0 + i < b_hi)
+                        p.c[(size_t)(b0 + i) * p.N + n] = __float2half_rn(__half2float(__float2half_rn(val[i])) + __half2float(res[i]));
+            } else {  // LLMB_EPI_ROPE_KV: the pair (even n, n + 1) sits in neighbouring lanes
+                float2 cs[R];
+                int pos[R];
+                size_t cache_row[R];
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const int b = min(b0 + i, b_hi - 1);
+                    cs[i] = is_v ? make_float2(1.0f, 0.0f) : __ldg(p.rope_cs + (size_t)b * half_dim + pair);
+                    pos[i] = kv_position(p, b, cache_row[i]);
+                }
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const float mine = __half2float(__float2half_rn(val[i]));
+                    const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
+                    __half out;
+                    if (is_v) {
+                        out = __float2half_rn(val[i]);
+                    } else {
+                        out = __float2half_rn((n & 1) ? __fmaf_rn(cs[i].y, other, __fmul_rn(cs[i].x, mine))
+                                                      : __fmaf_rn(cs[i].x, mine, -__fmul_rn(cs[i].y, other)));
+                    }
+                    if (valid && b0 + i < b_hi) {
+                        if (is_q) p.c[(size_t)(b0 + i) * p.n_q + n] = out;
+                        else if (pos[i] >= 0 && pos[i] < p.max_pos) (is_v ? p.v_cache : p.k_cache)[cache_row[i] * p.n_kv + local] = out;
+                    }
+                }
+            }
+        };
+        // CTA r of a cluster of S finishes activation rows r * nx/S ..: the loads of R rows x S slices go out together.
+        auto gather = [&](auto s_const) {
+            constexpr int S = decltype(s_const)::value, R = S >= 4 ? 4 : 8;  // eight with RoPE (S 4 as a rule): 3 us more of it, fetched cold
+            const int nb = nx / S, first = slice * nb, b_hi = min(first + nb, p.M);
+            uint32_t rbase[S];
+#pragma unroll
+            for (int z = 0; z < S; ++z) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbase[z]) : "r"(smem_u32(ring)), "r"(z));
+#pragma unroll 1
+            for (int b0 = first; b0 < b_hi; b0 += R) {
+                float t[(DUAL ? 2 : 1) * R][S], val[R], val2[R];
+#pragma unroll
+                for (int i = 0; i < (DUAL ? 2 : 1) * R; ++i) {
+                    const uint32_t off = (uint32_t)(((i / R * nx + min(b0 + i % R, b_hi - 1)) * kBM + nl) * 4);
+#pragma unroll
+                    for (int z = 0; z < S; ++z) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(t[i][z]) : "r"(rbase[z] + off));
+                }
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    val[i] = add_slices<S>(t[i], last_first);
+                    val2[i] = DUAL ? add_slices<S>(t[(DUAL ? R : 0) + i], last_first) : 0.0f;
+                }
+                finish(b0, b_hi, val, val2);
+            }
+        };
+        if (p.splits == 8) gather(std::integral_constant<int, 8>());
+        else if (p.splits == 4) gather(std::integral_constant<int, 4>());
+        else if (p.splits == 2) gather(std::integral_constant<int, 2>());
+        else {  // no split: straight from tensor memory
+#pragma unroll 1
+            for (int b0 = 0; b0 < p.M; b0 += 8) {
+                uint32_t v[8], u[8];
+                float val[8], val2[8];
+                tmem_ld8(taddr + b0, v);
+                if (DUAL) tmem_ld8(taddr + nx + b0, u);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    val[i] = __uint_as_float(v[i]);
+                    val2[i] = DUAL ? __uint_as_float(u[i]) : 0.0f;
+                }
+                finish(b0, p.M, val, val2);
             }
         }
     }
