@@ -1,8 +1,11 @@
 // Projections of long prompt blocks: C[M][N] = A[M][K] . B[N][K]^T as one persistent kernel, one CTA per SM, tiles of
 // 128 x 256 (SwiGLU: 128 gate + 128 up columns) handed out round robin.  Same arithmetic and epilogues as gemm_tc.cu.
 //
-// Bound: tensor pipe.  A 128 x 128 tile reads its two operands from shared memory at 128 bytes per cycle while it
-// multiplies, all that shared memory gives; at 128 x 256 the MMA needs 96, so the copies into the ring fit beside it.
+// Bound: tensor pipe, under the power cap.  A 128 x 128 tile reads its two operands from shared memory at 128 bytes per
+// cycle while it multiplies, all that shared memory gives; a 128 x 256 tile reads 96.  Prompt of 4096 tokens (8B shape)
+// 67.3 ms with 128 x 128 tiles, 60.0 with these: about 1.15 PFLOP/s in the projections.  CTA pairs (cta_group::2, 256 x 256
+// tiles, 64 bytes per cycle) gained 3 % from 3000 rows on and lost 2 % at 2000 to 2384; cutting the last wave's tiles along
+// K with FP32 parts in a workspace lost 6 % at 4096 rows and 20 % at 517 (a chain of L2 round trips per tile).
 // The accumulators are double-buffered (all 512 columns of tensor memory): the epilogue of one tile runs under the main
 // loop of the next, and the ring runs on across tiles.
 //
@@ -159,12 +162,14 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
 }
 
+// From 6/7 of a wave on: prompts of 1000 and 1024 tokens (o_proj and down_proj of the 8B shape: 128 tiles on 148 SMs) 16.6 ->
+// 15.6 ms against a whole wave; from half a wave on, 450 and 512 tokens lose 4 to 6 % and 800 gain 3.
 bool gemm_wide_takes(const LlmbGemmArgs *a) {
     if (a->tile_n != 0) return false;
     const int sms = sm_count_cached(), m_tiles = (a->m + kBM - 1) / kBM;
     const int tile_n = a->epilogue == LLMB_EPI_SWIGLU ? kWideN / 2 : kWideN;
     const long long wide = (long long)m_tiles * ((a->n + tile_n - 1) / tile_n);
-    return wide >= sms;
+    return wide * 7 >= 6LL * sms;
 }
 
 int launch_gemm_wide(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream) {
