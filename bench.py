@@ -283,8 +283,8 @@ def run_ours(args):
                              "frac_of_sustained": tf / peak_sust, "peak_sustained": peak_sust,
                              "flops": total, "projection_flops": proj, "attention_flops": attn,
                              "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst) / bf16_tflops_sustained"},
-                "path": "rows 0..n-2 as blocks of up to 1024 rows (tcgen05 projections, block attention), last row "
-                        "through the decode step (its 15 GB weight stream is inside this time)"}
+                "path": "blocks of up to 4096 rows (tcgen05 projections, block attention); the last row goes on to the "
+                        "logits"}
         if not args.quick:
             # decode behind the long prompt: cache rows 4097..4224 (the state the last prefill run left)
             cache.continue_greedy(3)

@@ -196,7 +196,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     // all of them: a CTA runs its epilogue once, so every instruction of it is fetched cold, and the fully unrolled form
     // (five epilogues x 32 rows) cost 5-19 us of instruction fetch per launch.  With a test per possible slice and
     // everything through shared memory it took 14 / 11 / 37 / 10 us of the four projections of a layer at 96 rows (last
-    // accumulator to last store); this form 14 / 10 / 10 / 8.
+    // accumulator to last store); this form 14 / 10 / 12 / 9.
     const int lane_group = (warp & 3) * 32;
     const int nl = lane_group + lane;
     const int n = n0 + nl;
