@@ -279,7 +279,8 @@ __device__ __forceinline__ float stage_dot(const unsigned char *base, size_t row
 // spilled in the projections as well (forms that held a whole K tile, or K across the barrier: 0.5-2 KB of spills and
 // 0.65 ms more per step, whatever they gained here).  So K comes in two halves, and at head_dim 128 two warps take the same
 // rows, each for 64 of V's dimensions.
-// 32-row tiles in shared memory with five CTA barriers each: 4.36 ms a step behind 4096 rows (8B shape); this form 3.24.
+// Against 32-row tiles in shared memory with five CTA barriers each (8B shape, ms per step behind 32 / 128 / 256 / 512 / 1024 /
+// 4096 rows): 3.00 / 3.00 / 2.98 / 3.00 / 3.41 / 4.14 -> 2.91 / 3.00 / 3.00 / 2.98 / 3.01 / 3.19.
 template <int HD>
 struct WarpAttn {
     static constexpr int KJ = HD / 32;        // chunks of 8 dimensions per lane and K row
@@ -340,7 +341,7 @@ __device__ __forceinline__ void attention_phase(const DsParams &p, const DsLayer
             float sc[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // (row gr, heads 2 gc, + 1), (row gr + 8, same heads)
             const uint4 *pk = reinterpret_cast<const uint4 *>(kb + (size_t)(t0 + gr) * n_kv) + gc;
             const bool in_a = t0 + gr < end, in_b = t0 + gr + 8 < end;
-#pragma unroll 1
+#pragma unroll
             for (int j = 0; j < W::KJ; j += 2) {
                 uint4 k[4];
 #pragma unroll
@@ -493,6 +494,34 @@ __device__ __forceinline__ void attention_phase(const DsParams &p, const DsLayer
             // (3) the partial outputs in batches of eight splits.
             const int n_used = min(p.n_splits, (len_total + p.split_len - 1) / p.split_len);
             const size_t gbase = (size_t)kvh * p.n_splits * G;
+            if (n_used <= 8) {
+                // few splits: a thread fetches its head's maxima and sums together with the partial outputs, one round
+                // trip and no barrier (the same operations in the same order as below)
+#pragma unroll 1
+                for (int o = tid; o < n_out; o += kDsConsumers) {
+                    const int hh = o / HD;
+                    float2 ml[8];
+                    float v[8], M = -INFINITY, num = 0.0f, den = 0.0f;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const size_t e = gbase + (size_t)u * G + hh;
+                        ml[u] = u < n_used ? __ldcg(reinterpret_cast<const float2 *>(&p.part_ml[e * 2])) : make_float2(-INFINITY, 0.0f);
+                        v[u] = u < n_used ? __ldcg(&p.part_o[e * HD + o % HD]) : 0.0f;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) M = fmaxf(M, ml[u].x);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        if (u < n_used) {
+                            const float wgt = ml[u].x == -INFINITY ? 0.0f : expf(ml[u].x - M);
+                            num = fmaf(wgt, v[u], num);
+                            den = fmaf(wgt, ml[u].y, den);
+                        }
+                    }
+                    p.attn[(size_t)kvh * n_out + o] = __float2half_rn(__fdiv_rn(num, den));
+                }
+                continue;
+            }
             float *m_all = sh.norm_buf[0];  // idle during attention: [split][head]
             float *l_all = sh.norm_buf[1];
             for (int e = tid; e < n_used * G; e += kDsConsumers) {
