@@ -1,5 +1,5 @@
-// Warp-level tensor-core helpers (mma.sync m16n8k16, FP16 in, FP32 accumulate) shared by the block attention
-// of the prompt phase (prefill.cu) and the decode attention (attn_decode.cu).
+// Warp-level tensor-core helpers (mma.sync m16n8k16, FP16 in, FP32 accumulate) shared by the decode attention
+// (attn_decode.cu) and the attention phase of the step kernel (decode_step.cu).
 #pragma once
 
 #include "common.cuh"

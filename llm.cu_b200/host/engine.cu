@@ -319,7 +319,7 @@ bool rows_shapes_ok(const Engine *e) {
            e->ffn % 128 == 0 && n_q % 64 == 0 && n_kv % 32 == 0 && e->vocab % 8 == 0;
 }
 
-// Blocks of up to 1024 rows: all of the model on this GPU.
+// Blocks of up to 4096 rows: all of the model on this GPU.
 bool prefill_supported(const Engine *e) { return e->tp_size == 1 && rows_shapes_ok(e); }
 
 // Tensor parallel: blocks of up to 32 rows through the weight-streaming projections with the all-reduce
