@@ -18,6 +18,7 @@ SOURCES = [
     "csrc/attn_decode.cu",
     "csrc/decode_step.cu",
     "csrc/gemm_tc.cu",
+    "csrc/gemm_mid.cu",
     "csrc/gemm_wide.cu",
     "csrc/gemm_smallm.cu",
     "csrc/prefill.cu",

@@ -237,6 +237,10 @@ int launch_gemm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t 
 // What every path of launch_gemm passes on of its arguments (gemm_tc.cu).
 int fill_gemm_params(GemmParams &p, const LlmbGemmArgs *a, int rows_per_seq);
 
+// The path for tiles that are one wave (gemm_mid.cu), and whether it takes this one.
+bool gemm_mid_takes(const LlmbGemmArgs *a);
+int launch_gemm_mid(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream);
+
 // The path for grids of many tiles (gemm_wide.cu), and whether it takes this one.
 bool gemm_wide_takes(const LlmbGemmArgs *a);
 int launch_gemm_wide(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream);

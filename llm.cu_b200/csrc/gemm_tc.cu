@@ -346,6 +346,7 @@ int llmb::launch_gemm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStr
     }
     // A handful of rows (batched decode): the weight-streaming kernel with the operands swapped
     if (small_m) return launch_gemm_smallm(a, rows_per_seq, pdl, stream);
+    if (gemm_mid_takes(a)) return launch_gemm_mid(a, rows_per_seq, pdl, stream);
     if (gemm_wide_takes(a)) return launch_gemm_wide(a, rows_per_seq, pdl, stream);
     // Small grids: with a workspace, 128-wide tiles and K split across CTAs until the SMs are covered
     // (every CTA then streams its own weights and only its slice of the activations); without one, the
