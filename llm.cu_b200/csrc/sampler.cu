@@ -16,15 +16,17 @@
 //              added in index order by one thread, 32 classes by a warp butterfly, the 32 warps' sums by another: the
 //              sum does not depend on how many CTAs share the work.
 //   order      only the first `want` entries can matter: top_k of them, or kSamplerMaxSelect where top_p is so close to 1
-//              that rounding may carry the prefix past the first top_k (see want_entries).  A radix select over the 64-bit
-//              key (bits of p, then inverted index, so that keys are unique and equal p keep index order) finds a key
-//              prefix that between `want` and kSamplerCap entries reach: usually the first histogram (exponent and 3
-//              mantissa bits of p) does.  Those entries go to CTA 0, which sorts them.
+//              that rounding may carry the prefix past the first top_k (see want_entries).  Whoever adds a class also keeps its
+//              largest t_i; as many entries as classes reach the `want`th largest of these, so the entries that do (usually not
+//              many more than wanted) go to CTA 0, which sorts them: one pass over the t_i without division or histogram.  Where
+//              more than kSamplerCap do, or more than half as many entries as classes are wanted, a radix select over the 64-bit key (bits
+//              of p, then inverted index, so that keys are unique and equal p keep index order) finds a key prefix that between
+//              `want` and kSamplerCap entries reach.
 //   chain      the reference's statements on CTA 0: the running sums are one thread's, in the reference's order; the
 //              divisions between them are elementwise and use all threads.
 // Taking the entries one at a time by a block-wide argmax on a single CTA (every round: two barriers, and the owner's
-// rescan of its entries) took 495 us a draw at top_k 50 over 128256 entries; this form takes 16 us (20 before short lists were ranked
-// by counting and the running sums lost their load and branch per entry).
+// rescan of its entries) took 495 us a draw at top_k 50 over 128256 entries; this form takes 14.4 us (18.5 with the general selection
+// for all; 20 before short lists were ranked by counting and the running sums lost their load and branch per entry).
 // Different from the host code: the sum of the t_i is a tree over classes, not a loop in index order, and expf is CUDA's,
 // so probabilities can differ from the host's by a few FP32 ulps; the token differs only if u lies within that distance
 // of a boundary between two entries.
@@ -42,6 +44,7 @@ constexpr int kRowsPerPass = kSamplerThreads / kClassesPerCta;         // 8 rows
 constexpr int kSamplerCap = 2048;                                      // entries that CTA 0 sorts at most
 constexpr int kSamplerSmemRows = 384;                                  // 192 KB of t_i per CTA: vocabularies up to 393216
 constexpr int kSamplerBins = 1024;
+constexpr int kLoadsInFlight = 16;                                     // per thread
 constexpr int kRankThreads = 4, kSamplerRankCap = kSamplerThreads / kRankThreads;  // up to 256 keys are ranked by counting
 
 struct SamplerParams {
@@ -98,6 +101,10 @@ __device__ __forceinline__ uint64_t sample_key(float pr, int i) {
     return ((uint64_t)__float_as_uint(pr) << 32) | (uint32_t)(0xffffffffu - (uint32_t)i);
 }
 
+// Bins of the classes' largest t_i: 16 to an octave, t_i of 2^-31 to 2^33; what lies outside is in the first or the last one.
+__device__ __forceinline__ int class_bin(float t) { return min(max((int)(__float_as_uint(t) >> 19) - (96 << 4), 0), kSamplerBins - 1); }
+__device__ __forceinline__ float class_bin_floor(int bin) { return bin == 0 ? 0.0f : __uint_as_float((uint32_t)(bin + (96 << 4)) << 19); }
+
 // Index of the first entry whose running sum (in order, one rounding per entry) satisfies `hit`, -1 if none does; `run` =
 // the running sum up to it (or of all n).  No probability is negative, so a sum of eight is looked at only if its last
 // running value hits: the chain is then one addition per entry, not a load, an addition and a branch.
@@ -128,6 +135,7 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     __shared__ int scan_s[32];
     __shared__ int bin_s, above_s, count_s;         // threshold bin, entries above it, entries from it on
     __shared__ int n_list;                          // CTA 0: entries collected
+    __shared__ int over_s;                          // more than the list takes
     __shared__ uint64_t list[kSamplerCap];          // CTA 0
     __shared__ float sel_p[kSamplerMaxSelect];
     __shared__ float sum_s;
@@ -138,34 +146,46 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     pdl_launch_dependents();
     pdl_wait();
 
+    // The classes' largest entries lead to the wanted ones only where these are fewer than the classes, and it pays where a class has
+    // many (us a draw at 4096 / 32768 / 128256 entries, top_k 50: 9.5 / 11.1 / 18.5 without, 10.0 / 10.3 / 14.4 with it).
+    const bool by_class = p.want <= kSamplerClasses / 2 && p.vocab > 8 * kSamplerClasses;
     // ---- t_i of this CTA's classes: thread = class cls, rows row0, row0 + 8, ... ----
     const int cls = (int)cta * kClassesPerCta + (tid & (kClassesPerCta - 1)), row0 = tid / kClassesPerCta;
     const int rows = (p.vocab + kSamplerClasses - 1) / kSamplerClasses;
     // element (row, class) of the vocabulary: t[row * t_stride + (class within the CTA)]
     float *t = p.in_smem ? t_smem : p.probs + (size_t)cta * kClassesPerCta;
     const int t_stride = p.in_smem ? kClassesPerCta : kSamplerClasses, col = tid & (kClassesPerCta - 1);
-    for (int base = row0; base < rows; base += 8 * kRowsPerPass) {
-        __half x[8];
+    for (int base = row0; base < rows; base += kLoadsInFlight * kRowsPerPass) {
+        __half x[kLoadsInFlight];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {  // eight loads in flight
+        for (int j = 0; j < kLoadsInFlight; ++j) {
             const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
             x[j] = row < rows && i < p.vocab ? p.logits[i] : __half(0.0f);
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < kLoadsInFlight; ++j) {
             const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
             if (row < rows && i < p.vocab) t[(size_t)row * t_stride + col] = expf(__fdiv_rn(__half2float(x[j]), p.temperature));
         }
     }
     if (tid < kSamplerBins) hist[tid] = 0;
-    if (tid == 0) n_list = 0;
+    if (tid == 0) {
+        n_list = 0;
+        bin_s = -1;
+        over_s = 0;
+    }
     __syncthreads();
     sampler_cluster_started_wait();
     if (tid < kClassesPerCta) {  // here col == tid
-        float local = 0.0f;
+        float local = 0.0f, most = 0.0f;
         const int n = cls < p.vocab ? (p.vocab - cls + kSamplerClasses - 1) / kSamplerClasses : 0;
 #pragma unroll 8
-        for (int row = 0; row < n; ++row) local += t[(size_t)row * t_stride + col];
+        for (int row = 0; row < n; ++row) {
+            const float v = t[(size_t)row * t_stride + col];
+            local += v;
+            most = fmaxf(most, v);
+        }
+        if (n > 0 && by_class) atomicAdd(&hist[class_bin(most)], 1);
         local = warp_sum(local);
         if (lane < kSamplerCtas)  // the same value in all lanes: lane c tells CTA c
             asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer_smem(&warp_sums[cta * (kClassesPerCta / 32) + warp], lane)), "f"(local) : "memory");
@@ -177,26 +197,20 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
         return;
     }
 
-    // ---- p_i, and a key prefix that enough entries reach ----
-    for (int row = row0; row < rows; row += kRowsPerPass) {
-        if (row * kSamplerClasses + cls >= p.vocab) break;
-        const float pr = __fdiv_rn(t[(size_t)row * t_stride + col], total);
-        t[(size_t)row * t_stride + col] = pr;
-        atomicAdd(&hist[__float_as_uint(pr) >> 20], 1);  // p <= 1: the bin is at most 0x3f8
-    }
-    uint64_t floor_key = 0;  // prefix of the keys that are taken, at `shift`
-    int shift = 52, need = p.want;
-    for (;;) {
-        sampler_cluster_sync();  // the histograms of all CTAs are complete
-        int cnt = 0;
+    // ---- the entries that can matter, from the classes' largest ones ----
+    // As many entries reach F as classes' largest ones do: F = the lower end of the bin that holds the `want`th largest of these.
+    // Division by the total keeps the order but may join neighbours, so whoever reaches F / total as a probability is taken; the
+    // division is left out where t_i is further below F than its rounding.
+    int inc, cnt;
+    auto count_down = [&]() {  // thread b holds bin 1023 - b of all CTAs: an inclusive scan counts the entries of that bin and all higher ones
+        cnt = 0;
 #pragma unroll
         for (int z = 0; z < kSamplerCtas; ++z) {
             int v;
             asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(peer_smem(&hist[kSamplerBins - 1 - tid], z)) : "memory");
             cnt += v;
         }
-        // thread b holds bin 1023 - b: an inclusive scan counts the entries of that bin and all higher ones
-        int inc = cnt;
+        inc = cnt;
 #pragma unroll
         for (int m = 1; m < 32; m <<= 1) {
             const int o = __shfl_up_sync(0xffffffffu, inc, m);
@@ -205,43 +219,86 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
         if (lane == 31) scan_s[warp] = inc;
         __syncthreads();
         inc += __reduce_add_sync(0xffffffffu, lane < warp ? scan_s[lane] : 0);
-        if (inc >= need && inc - cnt < need) {
-            bin_s = kSamplerBins - 1 - tid;
-            above_s = inc - cnt;
-            count_s = inc;
+    };
+    const uint32_t n_list0 = peer_smem(&n_list, 0), list0 = peer_smem(list, 0);
+    auto take = [&](uint64_t key) {
+        int at;
+        asm volatile("atom.relaxed.cluster.shared::cluster.add.s32 %0, [%1], 1;" : "=r"(at) : "r"(n_list0) : "memory");
+        if (at < kSamplerCap) {
+            asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(list0 + (uint32_t)at * 8), "l"(key) : "memory");
+        } else {
+            for (int z = 0; z < kSamplerCtas; ++z) asm volatile("st.shared::cluster.s32 [%0], 1;" ::"r"(peer_smem(&over_s, z)) : "memory");
         }
+    };
+    if (by_class) {
+        count_down();
+        if (inc >= p.want && inc - cnt < p.want) bin_s = kSamplerBins - 1 - tid;
         __syncthreads();
-        floor_key += (uint64_t)bin_s;
-        // entries above the bins of this level were counted out of `need` already: they are among the taken ones too
-        if (p.want - need + count_s <= kSamplerCap || shift == 0) break;
-        need -= above_s;
-        const int bits = shift >= 10 ? 10 : shift;
-        const int next = shift - bits;
-        sampler_cluster_sync();  // every CTA has read the histograms
-        hist[tid] = 0;
-        __syncthreads();
+    }
+    if (bin_s >= 0) {  // the same in all CTAs; else there are fewer classes than wanted entries
+        const float floor_t = class_bin_floor(bin_s), floor_p = __fdiv_rn(floor_t, total), near_t = floor_t * 0.999999f;
+#pragma unroll 4
+        for (int row = row0; row < rows; row += kRowsPerPass) {
+            const int i = row * kSamplerClasses + cls;
+            const float v = i < p.vocab ? t[(size_t)row * t_stride + col] : -1.0f;
+            if (v >= near_t) {
+                const float pr = __fdiv_rn(v, total);
+                if (pr >= floor_p) take(sample_key(pr, i));
+            }
+        }
+    }
+    if (by_class) sampler_cluster_sync();
+    if (bin_s < 0 || over_s) {  // too many reach F: the general way.  The same in every thread of the cluster
+        if (by_class) {
+            if (tid == 0) n_list = 0;
+            hist[tid] = 0;
+            __syncthreads();
+        }
+        // ---- p_i, and a key prefix that enough entries reach ----
+        for (int row = row0; row < rows; row += kRowsPerPass) {
+            if (row * kSamplerClasses + cls >= p.vocab) break;
+            const float pr = __fdiv_rn(t[(size_t)row * t_stride + col], total);
+            t[(size_t)row * t_stride + col] = pr;
+            atomicAdd(&hist[__float_as_uint(pr) >> 20], 1);  // p <= 1: the bin is at most 0x3f8
+        }
+        uint64_t floor_key = 0;  // prefix of the keys that are taken, at `shift`
+        int shift = 52, need = p.want;
+        for (;;) {
+            sampler_cluster_sync();  // the histograms of all CTAs are complete
+            count_down();
+            if (inc >= need && inc - cnt < need) {
+                bin_s = kSamplerBins - 1 - tid;
+                above_s = inc - cnt;
+                count_s = inc;
+            }
+            __syncthreads();
+            floor_key += (uint64_t)bin_s;
+            // entries above the bins of this level were counted out of `need` already: they are among the taken ones too
+            if (p.want - need + count_s <= kSamplerCap || shift == 0) break;
+            need -= above_s;
+            const int bits = shift >= 10 ? 10 : shift;
+            const int next = shift - bits;
+            sampler_cluster_sync();  // every CTA has read the histograms
+            hist[tid] = 0;
+            __syncthreads();
+            for (int row = row0; row < rows; row += kRowsPerPass) {
+                const int i = row * kSamplerClasses + cls;
+                if (i >= p.vocab) break;
+                const uint64_t key = sample_key(t[(size_t)row * t_stride + col], i);
+                if ((key >> shift) == floor_key) atomicAdd(&hist[(int)(key >> next) & ((1 << bits) - 1)], 1);
+            }
+            floor_key <<= bits;
+            shift = next;
+        }
+        // ---- the entries that reach it go to CTA 0 ----
         for (int row = row0; row < rows; row += kRowsPerPass) {
             const int i = row * kSamplerClasses + cls;
             if (i >= p.vocab) break;
             const uint64_t key = sample_key(t[(size_t)row * t_stride + col], i);
-            if ((key >> shift) == floor_key) atomicAdd(&hist[(int)(key >> next) & ((1 << bits) - 1)], 1);
+            if ((key >> shift) >= floor_key) take(key);
         }
-        floor_key <<= bits;
-        shift = next;
+        sampler_cluster_sync();
     }
-    // ---- the entries that reach it go to CTA 0 ----
-    const uint32_t n_list0 = peer_smem(&n_list, 0), list0 = peer_smem(list, 0);
-    for (int row = row0; row < rows; row += kRowsPerPass) {
-        const int i = row * kSamplerClasses + cls;
-        if (i >= p.vocab) break;
-        const uint64_t key = sample_key(t[(size_t)row * t_stride + col], i);
-        if ((key >> shift) >= floor_key) {
-            int at;
-            asm volatile("atom.relaxed.cluster.shared::cluster.add.s32 %0, [%1], 1;" : "=r"(at) : "r"(n_list0) : "memory");
-            if (at < kSamplerCap) asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(list0 + (uint32_t)at * 8), "l"(key) : "memory");
-        }
-    }
-    sampler_cluster_sync();
     if (cta != 0) return;
 
     // ---- descending order of the collected keys ----
