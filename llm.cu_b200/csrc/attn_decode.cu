@@ -495,7 +495,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     // quota: an equal share, but pieces no shorter than asked and never more than n_slots pieces per sequence
     // (a sequence of T tiles meets at most ceil(T / Q) + 1 groups, and Q >= ceil(longest / n_splits))
     int quota = (total + groups - 1) / groups;
-    quota = max(quota, max(p.min_tiles, (longest + p.n_splits - 1) / p.n_splits));
+    // Sequences of up to four tiles stay whole: a piece's tile takes 1 us, the merge of pieces 5.
+    quota = max(quota, max(longest <= 4 ? max(p.min_tiles, longest) : p.min_tiles, (longest + p.n_splits - 1) / p.n_splits));
     const int t_end = min((grp + 1) * quota, total);
     // the piece that starts at tile t of the group's run (t < t_end)
     auto piece_at = [&](int t, int &seq, int &tiles) {

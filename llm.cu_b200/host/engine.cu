@@ -96,7 +96,7 @@ struct Engine {
     int *bt_pos = nullptr, *bt_tok = nullptr, *bt_history = nullptr;  // [n_seqs], [n_seqs], [n_seqs][max_seq + 1]
     void *bt_attn_scratch = nullptr;
     int bt_max_splits = 0;
-    int bt_split_len = 256;                             // cache rows per attention CTA (a power of two, 32..512)
+    int bt_split_len = 0;                               // cache rows per attention CTA (a power of two, 32..512; 0: batch_split_len)
     std::vector<int> bt_len;                            // rows in the cache per sequence (host view)
     std::map<int, cudaGraphExec_t> bt_graphs;           // key: attention bucket
     // profiling aid: per-CTA stamps of every small-M projection of a step (cache_debug_rows_trace)
@@ -1153,6 +1153,11 @@ extern "C" int inference_continue(Llama3 *m, CudaCache *cache, int n_steps, int 
 // ---------------------------------------------------------------------------------------------
 namespace {
 
+// Cache rows per attention CTA where the caller has not said.  ms a step (8B) with 64 / 128 / 256 rows: 1 x 200 3.37 / 3.40 / 3.27 (fixed
+// splits; of several sequences those of up to 256 rows stay whole), 5 x 100 3.37 / 3.31 / 3.44, 5 x 333 3.59 / 3.46 / 3.59, 16 x 500
+// 3.79 / 3.76 / 3.88, 32 x 1024 4.42 / 4.39 / 4.43, 96 x 200 5.10 / 5.09 / 5.21.
+int batch_split_len(const Engine *e) { return e->bt_split_len > 0 ? e->bt_split_len : e->bt_seqs == 1 ? 256 : 128; }
+
 SplitPlan plan_batch_splits(int len, int split_len) {
     int bucket = 512;
     while (bucket < len) bucket <<= 1;
@@ -1214,7 +1219,7 @@ int enqueue_batch_step(Engine *e, const SplitPlan &sp) {
 
 // One batched step for sequences whose longest has `len` rows after it.
 int run_batch_step(Engine *e, int len) {
-    const SplitPlan sp = plan_batch_splits(len, e->bt_split_len);
+    const SplitPlan sp = plan_batch_splits(len, batch_split_len(e));
     if (int rc = ensure_prefill_buffers(e, e->bt_seqs, e->bt_seqs)) return rc;  // there already, unless a growth has failed
     e->launches += 2 + 7 * e->layers + 2 + (e->tp_size > 1 ? 1 : 0);
     if (!e->use_graph) return enqueue_batch_step(e, sp);
