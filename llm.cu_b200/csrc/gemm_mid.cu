@@ -7,10 +7,12 @@
 //
 // Bound: L2 to shared memory.  Per K step of 16 an SM loads (128 + nt) x 32 bytes, at 62 to 64 bytes a cycle, and the MMA takes
 // max(nt / 2, 32 + nt / 4) cycles (both measured): 64 + nt / 2 cycles a step, and no less than 120 with a stage of four steps, the
-// time of the waits, copies and MMAs of a stage.  So nt does not go below 96.  us at m = 200 / 384 / 517 rows (8B shape, from HBM) against
+// time of the waits, copies and MMAs of a stage.  So nt does not go below 96; where that leaves half of the SMs idle, K is cut in two
+// and the two CTAs of a tile are a cluster: each leaves the sums of half of the columns in its shared memory (the ring, free by
+// then) for the other, which adds them in slice order and finishes them.  Without slices, us at m = 200 / 384 / 517 rows (8B shape, from HBM) against
 // gemm_tc: QKV 45.1 / 47.0 / 55.7 -> 31.0 / 35.1 / 41.6, o_proj 32.9 / 33.7 / 36.8 -> 24.8 / 26.9 / 29.8, down_proj 65.7 / 96.0 / 101.8 -> 63.8 / 68.8 / 77.5
 // (launched one by one, 10 us of each are the launch).
-// K is summed in two accumulators, four up to 128 columns (all 512 columns of tensor memory), which the epilogue adds: tcgen05.mma
+// The K of a CTA is summed in two accumulators, four up to 128 columns (all 512 columns of tensor memory), which the epilogue adds: tcgen05.mma
 // truncates where it adds to its accumulator, an error that grows with the length of the chain.
 //
 //   warps 0, 10  TMA: 16 KB of weights / 128 bytes per row of the block to a stage
@@ -55,7 +57,9 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
     unsigned char *ring = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(mid_smem) + 1023) & ~uintptr_t(1023));
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int nt = p.nx, stages = p.stages, k_tiles = p.K / kBK;
+    const bool clustered = p.splits > 1;  // K in two halves, the two CTAs of a tile are a cluster along y
+    const int slice = clustered ? (int)cluster_cta_rank() : 0, kt0 = slice * (p.K / kBK) / p.splits;
+    const int nt = p.nx, stages = p.stages, k_tiles = (slice + 1) * (p.K / kBK) / p.splits - kt0;
     const uint32_t stage_bytes = mid_stage_bytes(nt);
     const uint32_t idesc = (1u << 4) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
     // row tiles vary fastest: the CTAs of a weight tile run together and it comes from HBM once
@@ -82,6 +86,43 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     pdl_launch_dependents();  // this CTA has its tensor memory (see gemm_tc.cu)
 
+    // of 16 columns: what this CTA finishes (the other half of them the cluster's other CTA)
+    const int groups = nt / 16, middle = (groups + 1) / 2;
+    const int own_begin = slice == 0 ? 0 : middle, own_end = !clustered || slice == 1 ? groups : middle;
+    const int lane_group = (warp & 3) * 32, side = (warp - 2) >> 2;
+    const uint32_t taddr = tmem + ((uint32_t)lane_group << 16);
+    float *sums = reinterpret_cast<float *>(ring);  // [column of the other half][weight row], once the ring is free
+    bool done = false;                              // the accumulators are complete
+    // sixteen columns of all accumulators
+    auto add = [&](int c, float (&v)[16]) {
+#pragma unroll 1
+        for (int b = 0; b < chains; ++b) {
+            uint32_t w[16];
+            tmem_ld16(taddr + b * acc_cols + c * 16, w);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = b == 0 ? __uint_as_float(w[i]) : v[i] + __uint_as_float(w[i]);
+        }
+    };
+    // Of two rows the even lanes take the first, the odd ones the second: features col, col + 1.
+    const bool odd = lane & 1;
+    const int col0 = n0 + lane_group, col = col0 + (lane & 30), half_dim = p.head_dim >> 1;
+    const bool is_q = col0 < p.n_q, is_v = col0 >= p.n_q + p.n_kv;
+    const int local = is_q ? col : (is_v ? col - p.n_q - p.n_kv : col - p.n_q), pair = half_dim > 0 ? (local >> 1) % half_dim : 0;
+    const bool residual = p.epilogue == LLMB_EPI_RESIDUAL, rope = p.epilogue == LLMB_EPI_ROPE_KV && !is_v;
+    const int own_middle = own_begin + (own_end - own_begin + 1) / 2;
+    const int c_begin = side == 0 ? own_begin : own_middle, c_end = side == 0 ? own_middle : own_end;
+    // What a group of rows needs besides the sums (residual: x, RoPE: y too) is asked for one group ahead.
+    float2 next[8];
+    auto ask = [&](int c) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int row = min(m0 + c * 16 + 2 * i + (odd ? 1 : 0), p.M - 1);
+            next[i] = make_float2(0.0f, 0.0f);
+            if (residual && col0 < p.N) next[i].x = __uint_as_float(__ldcg(reinterpret_cast<const unsigned int *>(p.c + (size_t)row * p.N + col)));
+            if (rope) next[i] = __ldg(p.rope_cs + (size_t)row * half_dim + pair);
+        }
+    };
+
     if (prior_status != 0) {
         pdl_wait();
     } else if (warp == 0 || warp == 10) {
@@ -103,7 +144,7 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             free = mid_peek(&empty_bar[s2], parity2);  // the answer comes while this stage is asked for
             if (mid_elect()) {
                 mbar_arrive_expect_tx(&full_bar[s], bytes);
-                tma_load_2d(base + (size_t)s * stage_bytes, map, kt * kBK, y, &full_bar[s]);
+                tma_load_2d(base + (size_t)s * stage_bytes, map, (kt0 + kt) * kBK, y, &full_bar[s]);
             }
             __syncwarp();
             s = s2;
@@ -143,47 +184,44 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (!ok && lane == 0) wind_down_mma(full_bar, stages, kt, min(kt + stages, k_tiles), &drain_bar);
     } else {
         // ---- epilogue ----
-        const int lane_group = (warp & 3) * 32, side = (warp - 2) >> 2, groups = nt / 16;
-        const int c_begin = side == 0 ? 0 : (groups + 1) / 2, c_end = side == 0 ? (groups + 1) / 2 : groups;  // of 16 columns
-        const uint32_t taddr = tmem + ((uint32_t)lane_group << 16);
-        // Of two rows the even lanes take the first, the odd ones the second: features col, col + 1.
-        const bool odd = lane & 1;
-        const int col0 = n0 + lane_group, col = col0 + (lane & 30), half_dim = p.head_dim >> 1;
-        const bool is_q = col0 < p.n_q, is_v = col0 >= p.n_q + p.n_kv;
-        const int local = is_q ? col : (is_v ? col - p.n_q - p.n_kv : col - p.n_q), pair = half_dim > 0 ? (local >> 1) % half_dim : 0;
-        const bool residual = p.epilogue == LLMB_EPI_RESIDUAL, rope = p.epilogue == LLMB_EPI_ROPE_KV && !is_v;
-        pdl_wait();  // the epilogue reads and writes global memory of earlier kernels
-        // What a group of rows needs besides the sums (residual: x, RoPE: y too) is asked for one group ahead.
-        float2 next[8];
-        auto ask = [&](int c) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int row = min(m0 + c * 16 + 2 * i + (odd ? 1 : 0), p.M - 1);
-                next[i] = make_float2(0.0f, 0.0f);
-                if (residual && col0 < p.N) next[i].x = __uint_as_float(__ldcg(reinterpret_cast<const unsigned int *>(p.c + (size_t)row * p.N + col)));
-                if (rope) next[i] = __ldg(p.rope_cs + (size_t)row * half_dim + pair);
-            }
-        };
-        ask(c_begin);
-        bool ok = mbar_wait_warp(&acc_bar, 0, p.status, 363, lane);
-        if (!ok) mbar_wait(&acc_bar, 0, nullptr, 0);
+        pdl_wait();  // it reads and writes global memory of earlier kernels
+        if (c_begin < c_end) ask(c_begin);
+        done = mbar_wait_warp(&acc_bar, 0, p.status, 363, lane);
+        if (!done) mbar_wait(&acc_bar, 0, nullptr, 0);
         // a wait of another warp that gave up has set the status word: the accumulators are incomplete
-        ok = __all_sync(0xffffffffu, ok && *reinterpret_cast<volatile int *>(p.status) == 0);
+        done = __all_sync(0xffffffffu, done && *reinterpret_cast<volatile int *>(p.status) == 0);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (clustered) {  // the other CTA's columns: through this one's shared memory
+            const int begin = slice == 0 ? middle : 0, end = slice == 0 ? groups : middle;
+#pragma unroll 1
+            for (int c = begin + side; c < end; c += 2) {
+                float v[16];
+                add(c, v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) sums[((c - begin) * 16 + i) * kBM + lane_group + lane] = v[i];
+            }
+        }
+    }
+    if (clustered) cluster_sync_all();  // both halves of K are there
+    if (warp >= 2 && warp < 10) {
+        uint32_t other_sums = 0;
+        if (clustered) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(other_sums) : "r"(smem_u32(sums)), "r"(slice ^ 1));
         // Not unrolled: a CTA runs its epilogue once, so every instruction of it is fetched cold.
 #pragma unroll 1
-        for (int c = c_begin; c < c_end && ok; ++c) {
+        for (int c = c_begin; c < c_end && done; ++c) {
             float2 now[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) now[i] = next[i];
             if (c + 1 < c_end) ask(c + 1);
             float v[16];
-#pragma unroll 1
-            for (int b = 0; b < chains; ++b) {
-                uint32_t w[16];
-                tmem_ld16(taddr + b * acc_cols + c * 16, w);
+            add(c, v);
+            if (clustered) {
+                float w[16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = b == 0 ? __uint_as_float(w[i]) : v[i] + __uint_as_float(w[i]);
+                for (int i = 0; i < 16; ++i)
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(w[i]) : "r"(other_sums + (uint32_t)(((c - own_begin) * 16 + i) * kBM + lane_group + lane) * 4));
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] += w[i];
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -216,25 +254,38 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (clustered) cluster_sync_all();  // no CTA leaves while the other may still read its sums
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
 }
 
-// Rows of a tile where all tiles are one wave of at least 3/8 of the SMs, 0 where they are not.  From 225 rows on gemm_wide.cu is
-// as fast or faster: prompts of 1000 / 1024 tokens (o_proj and down_proj in tiles of 256) 15.6 / 15.6 -> 15.9 / 16.2 ms with this
-// kernel, of 600 / 700 / 800 tokens 11.9 / 13.2 / 14.4 -> 10.6 / 12.1 / 13.6, of 129 / 200 / 300 / 517 6.98 / 7.06 / 8.80 / 11.4 -> 6.40 / 6.42 / 7.43 / 10.1.
-// Where gemm_tc.cu cuts K into three and more parts, its sums are in shorter chains than here: it keeps those.
-static int mid_tile_rows(int m, int n, int sms) {
-    const int w_tiles = (n + kBM - 1) / kBM, cuts = std::min(sms / w_tiles, (m + 95) / 96);
-    if (cuts < 1 || w_tiles * cuts * 8 < 3 * sms || w_tiles * ((m + 127) / 128) * 3 <= sms) return 0;
-    const int nt = ((m + cuts - 1) / cuts + 15) / 16 * 16;
-    return nt <= 224 ? nt : 0;
+// Rows of a tile and slices of K where all tiles are one wave of at least 3/8 of the SMs; 0 rows where they are not.  Of the cuts of
+// the rows and the one or two slices the pair whose CTAs take least time, a step of 16 at max(121, 64 + nt / 2) cycles.  Prompts of 129 /
+// 200 / 256 tokens without slices 6.40 / 6.42 / 6.57 ms, with them 5.39 / 5.60 / 5.85.
+// From 225 rows a tile on gemm_wide.cu is as fast or faster: prompts of 1000 / 1024 tokens (o_proj and down_proj in tiles of 256) 15.6 / 15.6 ->
+// 15.9 / 16.2 ms with this kernel.  Where gemm_tc.cu cuts K into three and more parts, its sums are in shorter chains than here: it
+// keeps those.
+static int mid_tile_rows(int m, int n, int k, int sms, int &splits) {
+    const int w_tiles = (n + kBM - 1) / kBM;
+    int best = 0, least = 0;
+    splits = 1;
+    if (w_tiles * ((m + 127) / 128) * 3 <= sms) return 0;
+    for (int s = 1; s <= (k / kBK >= 32 ? 2 : 1); ++s)
+        for (int cuts = 1; w_tiles * cuts * s <= sms && cuts <= (m + 95) / 96; ++cuts) {
+            const int nt = ((m + cuts - 1) / cuts + 15) / 16 * 16, cost = std::max(242, 128 + nt) / s;
+            if (nt > 224 || w_tiles * cuts * s * 8 < 3 * sms || (best && cost >= least)) continue;
+            best = nt;
+            least = cost;
+            splits = s;
+        }
+    return best;
 }
 
 bool gemm_mid_takes(const LlmbGemmArgs *a) {
-    return a->tile_n == 0 && a->epilogue != LLMB_EPI_SWIGLU && mid_tile_rows(a->m, a->n, sm_count_cached()) > 0;
+    int splits;
+    return a->tile_n == 0 && a->epilogue != LLMB_EPI_SWIGLU && mid_tile_rows(a->m, a->n, a->k, sm_count_cached(), splits) > 0;
 }
 
 int launch_gemm_mid(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream) {
@@ -242,7 +293,7 @@ int launch_gemm_mid(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStrea
     int rc;
     GemmParams p = {};
     if ((rc = fill_gemm_params(p, a, rows_per_seq))) return rc;
-    p.nx = mid_tile_rows(a->m, a->n, sm_count_cached());
+    p.nx = mid_tile_rows(a->m, a->n, a->k, sm_count_cached(), p.splits);
     p.stages = std::min(kMidMaxStages, (int)(kMidRing / mid_stage_bytes(p.nx)));
     if ((rc = make_map(&mw, a->b, a->n, a->k, kBM))) return rc;
     if ((rc = make_map(&mx, a->a, a->m, a->k, p.nx))) return rc;
@@ -250,7 +301,8 @@ int launch_gemm_mid(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStrea
     const size_t smem = (size_t)p.stages * mid_stage_bytes(p.nx) + 1024;
     static size_t attr_set[kMaxDevices] = {};
     LLMB_CUDA_OK(ensure_dynamic_smem(gemm_mid_kernel, attr_set, smem));
-    LLMB_CUDA_OK(launch_pdl(gemm_mid_kernel, dim3((unsigned)tiles), dim3(kMidThreads), smem, stream, pdl, mw, mx, p));
+    LLMB_CUDA_OK(launch_pdl_cluster(gemm_mid_kernel, dim3((unsigned)tiles, (unsigned)p.splits), dim3(kMidThreads), smem, stream, pdl,
+                                    dim3(1, (unsigned)p.splits, 1), mw, mx, p));
     return LLMB_OK;
 }
 

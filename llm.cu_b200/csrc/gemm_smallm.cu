@@ -39,18 +39,6 @@ constexpr uint32_t kWTileBytes = kBM * kBK * 2;           // 16 KB
 constexpr int kSmallMaxStages = 8;
 __host__ __device__ constexpr uint32_t small_stage_bytes(bool dual, int nx) { return (dual ? 2 : 1) * kWTileBytes + nx * kBK * 2; }
 
-__device__ __forceinline__ uint32_t cluster_cta_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-
-// Every thread of every CTA of the cluster arrives; returns when all have (a hardware barrier: no spin of ours).
-__device__ __forceinline__ void cluster_sync_all() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-
 // The sum of S slices' partial sums in slice order.
 template <int S>
 __device__ __forceinline__ float add_slices(const float (&t)[S]) {

@@ -1,5 +1,5 @@
 """The one-wave projection kernel of middling blocks (gemm_mid.cu) at its edges: the fewest rows, tiles of 16 columns more or less
-than the rows need, the last tile nearly empty, one K step, K steps that do not divide among the accumulators (two and four of them), the
+than the rows need, the last tile nearly empty, K in two slices (from 2048 on, also of odd lengths), one K step, K steps that do not divide among the accumulators (two and four of them), the
 most rows it takes and one more.  Against float64, tolerances as in test_gpu_prefill.py."""
 import numpy as np
 import pytest
@@ -18,7 +18,7 @@ def _need_gpu():
 
 
 @pytest.mark.parametrize("m,n,k", [(129, 4096, 64), (129, 4096, 320), (192, 4096, 4096), (193, 6144, 448), (145, 18816, 128), (224, 18944, 192),
-                                   (225, 18944, 64), (384, 4736, 1024), (385, 4096, 576), (517, 4096, 704), (896, 4096, 128), (897, 4096, 128)])
+                                   (225, 18944, 64), (384, 4736, 1024), (385, 4096, 576), (256, 4096, 2048), (257, 4096, 2112), (448, 4096, 2048), (200, 6144, 2176), (449, 4096, 2048), (517, 4096, 704), (896, 4096, 128), (897, 4096, 128)])
 def test_store_and_residual(pkg, oracle, m, n, k):
     a, b = mats(oracle, m, n, k, 50)
     da, db = dev(a), dev(b)
@@ -37,7 +37,7 @@ def test_store_and_residual(pkg, oracle, m, n, k):
                       abs_tol=(np.abs(acc) + np.abs(want)) * 2.0 ** -10 + tc_tol(acc, k))
 
 
-@pytest.mark.parametrize("m,nqh,nkvh,hd,k,batched", [(129, 32, 8, 128, 192, False), (300, 32, 8, 128, 64, True), (517, 20, 6, 128, 128, False), (250, 48, 12, 64, 320, False)])
+@pytest.mark.parametrize("m,nqh,nkvh,hd,k,batched", [(129, 32, 8, 128, 192, False), (200, 32, 8, 128, 2112, False), (210, 28, 6, 128, 2048, True), (300, 32, 8, 128, 64, True), (517, 20, 6, 128, 128, False), (250, 48, 12, 64, 320, False)])
 def test_rope_kv(pkg, oracle, m, nqh, nkvh, hd, k, batched):
     """Rows of one sequence, and one row of each of m sequences (row_pos)."""
     n_q, n_kv, pos0, max_pos = nqh * hd, nkvh * hd, 5, (16 if batched else m + 3)   # not batched: the last rows lie past the cache
