@@ -233,7 +233,8 @@ int cache_sample_next_token_device(CudaCache *cache, float temperature, int top_
  *   cache_batch_greedy   n_steps steps with the greedy tokens fed back on the device, no host round trip;
  *                        out_tokens [n_seqs][n_steps], ms = CUDA-event time of the steps */
 int cache_batch_init(CudaCache *cache, int n_seqs);
-/* Cache rows per attention CTA of the batched step (a power of two, 32..512; default 256). */
+/* Cache rows per attention CTA of the batched step (a power of two, 32..512), from now on.  While it has not been called: 128,
+ * and no fewer than the longest sequence has while that is at most 256; 256 for a batch of one sequence. */
 int cache_batch_set_split_len(CudaCache *cache, int split_len);
 int cache_batch_prefill(CudaCache *cache, const int *tokens, int n_tokens);
 int cache_batch_step(CudaCache *cache, const int *tokens, uint16_t *h_logits, int *next_tokens);

@@ -144,8 +144,9 @@ int llmb_attn_decode(const uint16_t *d_q, const uint16_t *d_k_cache, const uint1
 /* Batched decode: one new token for each of n_seqs sequences in one launch.  With 2..256 sequences */
 /* the launch is one wave of CTAs that share the 64-row tiles of all (sequence, KV head) pairs      */
 /* evenly, whatever the mix of lengths (read from pos on the device, so a captured launch stays      */
-/* valid as the sequences grow); a pair is cut into at most n_splits + 1 pieces of at least         */
-/* split_len rows, merged in piece order by the last CTA of the pair to finish.                      */
+/* valid as the sequences grow): the CTAs of one KV head take equal shares of at least split_len     */
+/* rows, so that a pair is cut into at most n_splits + 1 pieces, merged in piece order by the last   */
+/* CTA of the pair to finish.                                                                        */
 /*   q, out   : [n_seqs][n_q_heads * head_dim];  pos : device [n_seqs], position of each new token  */
 /*   k_cache  : [n_seqs][seq_stride_rows][n_kv_heads * head_dim] (this layer), likewise v_cache      */
 /*   n_splits * split_len must cover the longest sequence; scratch as below, counters zero.          */

@@ -60,8 +60,9 @@ struct AttnParams {
     unsigned long long *trace;  // optional profiling aid: [CTA][8] global-timer stamps (llmb_attn_decode_trace)
     int *status;                // device status word: a wait that runs out records its code there
     // balanced != 0 (several sequences): 1-D grid, tiles shared evenly; n_slots = n_splits + 1 partial slots per
-    // (sequence, KV head); a piece is at least min_tiles tiles long
-    int balanced, n_seqs, n_slots, min_tiles;
+    // (sequence, KV head); a group's share is at least min_tiles tiles, and the longest sequence if that has no more than
+    // whole_tiles (0: the caller has chosen the length of a piece)
+    int balanced, n_seqs, n_slots, min_tiles, whole_tiles;
     int seq_rows;  // batched: cache rows per sequence (seq_stride = seq_rows * n_kv_heads * head_dim)
 };
 
@@ -492,11 +493,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     const int g = (int)blockIdx.x % p.n_kv_heads, grp = (int)blockIdx.x / p.n_kv_heads;
     if (grp >= groups) return;
     const int total = pre_s[p.n_seqs];
-    // quota: an equal share, but pieces no shorter than asked and never more than n_slots pieces per sequence
+    // quota Q: an equal share, but no shorter than asked and never more than n_slots pieces per sequence
     // (a sequence of T tiles meets at most ceil(T / Q) + 1 groups, and Q >= ceil(longest / n_splits))
     int quota = (total + groups - 1) / groups;
-    // Sequences of up to four tiles stay whole: a piece's tile takes 1 us, the merge of pieces 5.
-    quota = max(quota, max(longest <= 4 ? max(p.min_tiles, longest) : p.min_tiles, (longest + p.n_splits - 1) / p.n_splits));
+    quota = max(quota, max(p.min_tiles, (longest + p.n_splits - 1) / p.n_splits));
+    // Where all sequences are short, Q is no less than the longest (a piece's tile takes 1 us, the merge of pieces 5): equal
+    // ones are then whole where the equal share is smaller; a larger one, or unequal lengths, still cut those on a multiple of Q.
+    if (longest <= p.whole_tiles) quota = max(quota, longest);
     const int t_end = min((grp + 1) * quota, total);
     // the piece that starts at tile t of the group's run (t < t_end)
     auto piece_at = [&](int t, int &seq, int &tiles) {
@@ -595,7 +598,7 @@ extern "C" int llmb_attn_decode_trace(void *d_trace) {
 static int attn_decode_impl(const uint16_t *d_q, const uint16_t *d_k_cache, const uint16_t *d_v_cache, const int32_t *d_pos,
                             int n_seqs, size_t seq_stride_elems, int n_q_heads, int n_kv_heads, int head_dim, int n_splits,
                             int split_len, uint16_t *d_out, void *d_scratch, int use_pdl, llmb_stream_t stream_,
-                            bool batch_scratch = false) {
+                            bool batch_scratch = false, int whole_tiles = 0) {
     using namespace llmb;
     if (!d_q || !d_k_cache || !d_v_cache || !d_pos || !d_out || !d_scratch) return LLMB_ERR_INVALID;
     if (n_kv_heads <= 0 || n_q_heads % n_kv_heads || n_splits <= 0 || split_len <= 0 || n_seqs <= 0 || n_seqs > 65535)
@@ -615,6 +618,7 @@ static int attn_decode_impl(const uint16_t *d_q, const uint16_t *d_k_cache, cons
     p.n_seqs = n_seqs;
     p.n_slots = n_splits + (batch_scratch ? 1 : 0);
     p.min_tiles = split_len / kTile > 0 ? split_len / kTile : 1;
+    p.whole_tiles = whole_tiles;
     if (p.balanced && !batch_scratch) p.balanced = 0;
     p.counters = reinterpret_cast<int *>(sc);
     sc += attn_counters_bytes(n_kv_heads * n_seqs);
@@ -667,9 +671,16 @@ extern "C" int llmb_attn_decode_batch(const uint16_t *d_q, const uint16_t *d_k_c
                                       const int32_t *d_pos, int n_seqs, size_t seq_stride_rows, int n_q_heads, int n_kv_heads,
                                       int head_dim, int n_splits, int split_len, uint16_t *d_out, void *d_scratch, int use_pdl,
                                       llmb_stream_t stream_) {
+    return llmb::launch_attn_decode_batch(d_q, d_k_cache, d_v_cache, d_pos, n_seqs, seq_stride_rows, n_q_heads, n_kv_heads, head_dim, n_splits,
+                                          split_len, 0, d_out, d_scratch, use_pdl, stream_);
+}
+
+int llmb::launch_attn_decode_batch(const uint16_t *d_q, const uint16_t *d_k_cache, const uint16_t *d_v_cache, const int32_t *d_pos, int n_seqs,
+                                   size_t seq_stride_rows, int n_q_heads, int n_kv_heads, int head_dim, int n_splits, int split_len,
+                                   int whole_rows, uint16_t *d_out, void *d_scratch, int use_pdl, llmb_stream_t stream_) {
     if (n_kv_heads <= 0 || head_dim <= 0) return LLMB_ERR_INVALID;
     return attn_decode_impl(d_q, d_k_cache, d_v_cache, d_pos, n_seqs, seq_stride_rows * (size_t)n_kv_heads * head_dim, n_q_heads,
-                            n_kv_heads, head_dim, n_splits, split_len, d_out, d_scratch, use_pdl, stream_, true);
+                            n_kv_heads, head_dim, n_splits, split_len, d_out, d_scratch, use_pdl, stream_, true, whole_rows / kTile);
 }
 
 // ---------------------------------------------------------------------------------------

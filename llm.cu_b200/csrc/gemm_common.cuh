@@ -261,6 +261,12 @@ int launch_gemm_wide(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStre
 constexpr int kSmallM = 128;
 int launch_gemm_smallm(const LlmbGemmArgs *a, int rows_per_seq, bool pdl, cudaStream_t stream);
 
+// llmb_attn_decode_batch where no caller has chosen the length of a piece: pieces of `split_len` rows, but no shorter than the
+// longest sequence if that has at most `whole_rows` (attn_decode.cu).
+int launch_attn_decode_batch(const uint16_t *d_q, const uint16_t *d_k_cache, const uint16_t *d_v_cache, const int32_t *d_pos, int n_seqs,
+                             size_t seq_stride_rows, int n_q_heads, int n_kv_heads, int head_dim, int n_splits, int split_len,
+                             int whole_rows, uint16_t *d_out, void *d_scratch, int use_pdl, llmb_stream_t stream);
+
 // Causal attention of `len` new rows of each of n_seqs sequences (attn_prefill.cu); the caches of consecutive
 // sequences are seq_stride elements apart, q and out are [n_seqs * len][n_q_heads * head_dim].
 int launch_attn_prefill(const __half *q, const __half *k_cache, const __half *v_cache, int n_seqs, size_t seq_stride, int len, int pos0,

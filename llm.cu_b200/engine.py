@@ -191,7 +191,8 @@ class Cache:
         self.n_seqs = int(n_seqs)
 
     def batch_set_split_len(self, split_len):
-        """Cache rows per attention CTA of the batched step (a power of two, 32..512)."""
+        """Cache rows per attention CTA of the batched step (a power of two, 32..512); by itself the engine takes 128, no fewer
+        than the longest sequence has while that is at most 256, and 256 for a batch of one."""
         check(lib.cache_batch_set_split_len(self.ptr, int(split_len)), "cache_batch_set_split_len")
 
     def batch_prefill(self, prompts):

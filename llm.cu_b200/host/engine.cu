@@ -1156,6 +1156,7 @@ namespace {
 // Cache rows per attention CTA where the caller has not said.  ms a step (8B) with 64 / 128 / 256 rows: 1 x 200 3.37 / 3.40 / 3.27 (fixed
 // splits; of several sequences those of up to 256 rows stay whole), 5 x 100 3.37 / 3.31 / 3.44, 5 x 333 3.59 / 3.46 / 3.59, 16 x 500
 // 3.79 / 3.76 / 3.88, 32 x 1024 4.42 / 4.39 / 4.43, 96 x 200 5.10 / 5.09 / 5.21.
+constexpr int kBatchWholeRows = 256;  // then also: no piece shorter than the longest sequence, if that has no more rows than this
 int batch_split_len(const Engine *e) { return e->bt_split_len > 0 ? e->bt_split_len : e->bt_seqs == 1 ? 256 : 128; }
 
 SplitPlan plan_batch_splits(int len, int split_len) {
@@ -1193,8 +1194,8 @@ int enqueue_batch_step(Engine *e, const SplitPlan &sp) {
         g.k_cache = u16w(kl); g.v_cache = u16w(vl);
         g.row_pos = e->bt_pos; g.seq_stride = e->max_seq; g.max_pos = e->max_seq;
         if ((rc = launch_gemm(&g, 0, e->use_pdl, s))) return rc;
-        if ((rc = llmb_attn_decode_batch(u16(e->pf_q), u16(kl), u16(vl), e->bt_pos, B, (size_t)e->max_seq, e->nq, e->nkv, e->hd,
-                                         sp.n_splits, sp.split_len, u16w(e->pf_attn), e->bt_attn_scratch, pdl, s)))
+        if ((rc = launch_attn_decode_batch(u16(e->pf_q), u16(kl), u16(vl), e->bt_pos, B, (size_t)e->max_seq, e->nq, e->nkv, e->hd, sp.n_splits,
+                                           sp.split_len, e->bt_split_len > 0 ? 0 : kBatchWholeRows, u16w(e->pf_attn), e->bt_attn_scratch, pdl, s)))
             return rc;
         if ((rc = row_parallel_projection(e, e->pf_attn, L->self_attn_o_proj->d_fp16_tensor, B, n_q,
                                           L->post_attention_layernorm->d_fp16_tensor, xi)))
