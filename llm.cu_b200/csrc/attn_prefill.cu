@@ -358,6 +358,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll 1
             for (int q = 0; q < HD / 32 && ok; ++q) {
                 uint32_t o[32];
+                __syncwarp();  // see tmem_ld32
                 tmem_ld32(to + q * 32, o);
                 if (i < p.len) {
 #pragma unroll

@@ -107,7 +107,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, i
     if (lane == 0) ok = mbar_wait(bar, parity, status, code) ? 1 : 0;
     ok = __shfl_sync(0xffffffffu, ok, 0);
     if (ok && lane != 0) ok = mbar_wait(bar, parity, status, code) ? 1 : 0;  // already complete: returns at once
-    return ok != 0;
+    return __all_sync(0xffffffffu, ok != 0);  // the same in all lanes, and these together again
 }
 
 // 1-D bulk copy global -> shared, completion counted in bytes on an mbarrier.  Source,

@@ -88,6 +88,9 @@ static __device__ __noinline__ void wind_down_mma(uint64_t *full_bar, int stages
     mbar_wait(drain_bar, 0, nullptr, 0);
 }
 
+// Tensor-memory loads are one instruction of a converged warp.  An epilogue that comes to one from masked stores, a `continue` for
+// rows past the end or a wait that each lane polls for itself joins the warp first (__syncwarp or a vote), instead of leaving it
+// to where the compiler brings the lanes together again.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "

@@ -209,6 +209,7 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // Not unrolled: a CTA runs its epilogue once, so every instruction of it is fetched cold.
 #pragma unroll 1
         for (int c = c_begin; c < c_end && done; ++c) {
+            __syncwarp();  // see tmem_ld32; before the loads below, which it would wait for
             float2 now[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) now[i] = next[i];

@@ -205,6 +205,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll 1
             for (int b0 = 0; b0 < (DUAL ? 2 : 1) * nx; b0 += 32) {
                 uint32_t v[32];
+                __syncwarp();  // see tmem_ld32
                 tmem_ld32(taddr + b0, v);
 #pragma unroll
                 for (int b = 0; b < 32; ++b) red_own[(b0 + b) * kBM + nl] = v[b];
@@ -314,6 +315,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             for (int b0 = 0; b0 < p.M; b0 += 8) {
                 uint32_t v[8], u[8];
                 float val[8], val2[8];
+                __syncwarp();  // see tmem_ld32
                 tmem_ld8(taddr + b0, v);
                 if (DUAL) tmem_ld8(taddr + nx + b0, u);
 #pragma unroll

@@ -152,6 +152,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const bool two_chains = !DUAL && kt_end - kt_begin > 1;
         // 32 columns of the accumulator, the two chains added; warp-collective
         auto load_acc = [&](uint32_t taddr, uint32_t (&v)[32]) {
+            __syncwarp();  // see tmem_ld32
             if (!two_chains) {
                 tmem_ld32(taddr, v);
                 return;
@@ -179,6 +180,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         reinterpret_cast<uint4 *>(mine + c * 32)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
                 }
                 if (DUAL) {
+                    __syncwarp();
                     tmem_ld32(taddr + kBN, v);
                     if (row_ok) {
 #pragma unroll

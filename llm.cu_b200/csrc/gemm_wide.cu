@@ -163,6 +163,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             release(0);
             if (chains > 1 && !wait_acc(1, n)) break;
             auto add_second = [&](int g) {
+                __syncwarp();  // see tmem_ld32
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     uint32_t w[16];
