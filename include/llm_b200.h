@@ -324,7 +324,9 @@ float llmb_sampler_uniform(uint64_t seed, uint64_t draw);
 /* 1024 entries: top_k (after clamping to vocab) above that returns LLMB_ERR_UNSUPPORTED.            */
 /*   scratch   : llmb_sample_scratch_bytes(vocab) bytes, 256-byte aligned; its first int32 is the     */
 /*               result code of the last call: 0 ok, 1 expf overflow, 2 the top-p prefix ran past    */
-/*               1024 entries (token_out is -1 in both cases: use the host sampler for that step)    */
+/*               1024 entries (token_out is -1 in both cases: use the host sampler for that step);   */
+/*               profiling aid, where it is 0: the second is the number of entries that were ordered, */
+/*               the third 1 if the selection by classes found them (0: the radix select)             */
 /*   token_out : the sampled id; if pos and history are given, history[*pos] = id as well (the       */
 /*               position the decode step has already advanced to: the next step then feeds it)     */
 size_t llmb_sample_scratch_bytes(int vocab);

@@ -19,17 +19,19 @@
 //              that rounding may carry the prefix past the first top_k (see want_entries).  Whoever adds a class also keeps its
 //              largest t_i; as many entries as classes reach the `want`th largest of these, so the entries that do (usually not
 //              many more than wanted) go to CTA 0, which sorts them: one pass over the t_i without division or histogram.  Where
-//              more than kSamplerCap do, or more than half as many entries as classes are wanted, a radix select over the 64-bit key (bits
-//              of p, then inverted index, so that keys are unique and equal p keep index order) finds a key prefix that between
-//              `want` and kSamplerCap entries reach.
+//              nearly all classes or more than kSamplerCap entries do, or more than half as many entries as classes are wanted, a radix
+//              select over the 64-bit key (bits of p, then inverted index, so that keys are unique and equal p keep index order)
+//              finds a key prefix that between `want` and kSamplerCap entries reach.
 //   chain      the reference's statements on CTA 0: the running sums are one thread's, in the reference's order; the
 //              divisions between them are elementwise and use all threads.
 // Taking the entries one at a time by a block-wide argmax on a single CTA (every round: two barriers, and the owner's
-// rescan of its entries) took 495 us a draw at top_k 50 over 128256 entries; this form takes 14.4 us (18.5 with the general selection
-// for all; 20 before short lists were ranked by counting and the running sums lost their load and branch per entry).
+// rescan of its entries) took 495 us a draw at top_k 50 over 128256 entries; this form takes 14.4 us at any temperature (18.5 with the radix
+// select for all; 20 before short lists were ranked by counting and the running sums lost their load and branch per entry).
 // Different from the host code: the sum of the t_i is a tree over classes, not a loop in index order, and expf is CUDA's,
 // so probabilities can differ from the host's by a few FP32 ulps; the token differs only if u lies within that distance
 // of a boundary between two entries.
+#include <type_traits>
+
 #include "common.cuh"
 #include "../../include/llm_b200_synth.h"
 
@@ -44,7 +46,8 @@ constexpr int kRowsPerPass = kSamplerThreads / kClassesPerCta;         // 8 rows
 constexpr int kSamplerCap = 2048;                                      // entries that CTA 0 sorts at most
 constexpr int kSamplerSmemRows = 384;                                  // 192 KB of t_i per CTA: vocabularies up to 393216
 constexpr int kSamplerBins = 1024;
-constexpr int kLoadsInFlight = 16;                                     // per thread
+constexpr int kClassBinWords = 1024;                                   // 4096 bins of the classes' largest t_i
+constexpr int kClassesListed = 880;  // classes whose largest entry reaches the floor, at most, for the list to be tried (see sample_kernel)
 constexpr int kRankThreads = 4, kSamplerRankCap = kSamplerThreads / kRankThreads;  // up to 256 keys are ranked by counting
 
 struct SamplerParams {
@@ -54,7 +57,7 @@ struct SamplerParams {
     int *pos;       // optional: history[*pos] = token (the position the decode step has already advanced to)
     int *history;
     int history_len;
-    int *result;    // 0 ok, 1 overflow, 2 prefix longer than kSamplerMaxSelect
+    int *result;    // 0 ok, 1 overflow, 2 prefix longer than kSamplerMaxSelect; then, where it is 0: entries ordered, 1 if the classes led to them
     int vocab, top_k;
     int want;       // entries of the order that may be needed, top_k <= want <= kSamplerMaxSelect
     int in_smem;    // t_i in shared memory (else in probs)
@@ -101,9 +104,10 @@ __device__ __forceinline__ uint64_t sample_key(float pr, int i) {
     return ((uint64_t)__float_as_uint(pr) << 32) | (uint32_t)(0xffffffffu - (uint32_t)i);
 }
 
-// Bins of the classes' largest t_i: 16 to an octave, t_i of 2^-31 to 2^33; what lies outside is in the first or the last one.
-__device__ __forceinline__ int class_bin(float t) { return min(max((int)(__float_as_uint(t) >> 19) - (96 << 4), 0), kSamplerBins - 1); }
-__device__ __forceinline__ float class_bin_floor(int bin) { return bin == 0 ? 0.0f : __uint_as_float((uint32_t)(bin + (96 << 4)) << 19); }
+// Bins of the classes' largest t_i: 16 to an octave over all of FP32, so that the scale of the logits and the temperature do not
+// matter.  A CTA has 128 classes: a bin's count is a byte, four bins a word.
+__device__ __forceinline__ int class_bin(float t) { return (int)(__float_as_uint(t) >> 19); }
+__device__ __forceinline__ float class_bin_floor(int bin) { return __uint_as_float((uint32_t)bin << 19); }
 
 // Index of the first entry whose running sum (in order, one rounding per entry) satisfies `hit`, -1 if none does; `run` =
 // the running sum up to it (or of all n).  No probability is negative, so a sum of eight is looked at only if its last
@@ -132,10 +136,11 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     extern __shared__ float t_smem[];               // [rows][128] t_i, then p_i, of this CTA's classes
     __shared__ float warp_sums[32];                 // of all CTAs
     __shared__ int hist[kSamplerBins];
+    __shared__ unsigned int class_hist[kClassBinWords];
     __shared__ int scan_s[32];
     __shared__ int bin_s, above_s, count_s;         // threshold bin, entries above it, entries from it on
     __shared__ int n_list;                          // CTA 0: entries collected
-    __shared__ int over_s;                          // more than the list takes
+    __shared__ int over_s;                          // the list is full
     __shared__ uint64_t list[kSamplerCap];          // CTA 0
     __shared__ float sel_p[kSamplerMaxSelect];
     __shared__ float sum_s;
@@ -147,7 +152,7 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     pdl_wait();
 
     // The classes' largest entries lead to the wanted ones only where these are fewer than the classes, and it pays where a class has
-    // many (us a draw at 4096 / 32768 / 128256 entries, top_k 50: 9.5 / 11.1 / 18.5 without, 10.0 / 10.3 / 14.4 with it).
+    // many (us a draw at 32768 / 65536 / 128256 entries, top_k 50: 11.0 / 12.6 / 18.5 without, 10.3 / 12.3 / 14.4 with it; over 4096 it lost 0.5).
     const bool by_class = p.want <= kSamplerClasses / 2 && p.vocab > 8 * kSamplerClasses;
     // ---- t_i of this CTA's classes: thread = class cls, rows row0, row0 + 8, ... ----
     const int cls = (int)cta * kClassesPerCta + (tid & (kClassesPerCta - 1)), row0 = tid / kClassesPerCta;
@@ -155,23 +160,30 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     // element (row, class) of the vocabulary: t[row * t_stride + (class within the CTA)]
     float *t = p.in_smem ? t_smem : p.probs + (size_t)cta * kClassesPerCta;
     const int t_stride = p.in_smem ? kClassesPerCta : kSamplerClasses, col = tid & (kClassesPerCta - 1);
-    for (int base = row0; base < rows; base += kLoadsInFlight * kRowsPerPass) {
-        __half x[kLoadsInFlight];
+    auto exponentials = [&](auto loads) {  // so many of a thread's loads in flight
+        constexpr int L = decltype(loads)::value;
+        for (int base = row0; base < rows; base += L * kRowsPerPass) {
+            __half x[L];
 #pragma unroll
-        for (int j = 0; j < kLoadsInFlight; ++j) {
-            const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
-            x[j] = row < rows && i < p.vocab ? p.logits[i] : __half(0.0f);
-        }
+            for (int j = 0; j < L; ++j) {
+                const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
+                x[j] = row < rows && i < p.vocab ? p.logits[i] : __half(0.0f);
+            }
 #pragma unroll
-        for (int j = 0; j < kLoadsInFlight; ++j) {
-            const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
-            if (row < rows && i < p.vocab) t[(size_t)row * t_stride + col] = expf(__fdiv_rn(__half2float(x[j]), p.temperature));
+            for (int j = 0; j < L; ++j) {
+                const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
+                if (row < rows && i < p.vocab) t[(size_t)row * t_stride + col] = expf(__fdiv_rn(__half2float(x[j]), p.temperature));
+            }
         }
-    }
-    if (tid < kSamplerBins) hist[tid] = 0;
+    };
+    // sixteen: eight took up to 2 us more over 128256 entries.  One where a thread has no second row: 18.9 us against 19.5 over 4096
+    // entries at top_k 500, 21.2 against 22.8 over 8192
+    if (rows <= kRowsPerPass) exponentials(std::integral_constant<int, 1>());
+    else exponentials(std::integral_constant<int, 16>());
+    hist[tid] = 0;
+    class_hist[tid] = 0;
     if (tid == 0) {
         n_list = 0;
-        bin_s = -1;
         over_s = 0;
     }
     __syncthreads();
@@ -185,7 +197,10 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
             local += v;
             most = fmaxf(most, v);
         }
-        if (n > 0 && by_class) atomicAdd(&hist[class_bin(most)], 1);
+        if (n > 0 && by_class) {
+            const int bin = class_bin(most);
+            atomicAdd(&class_hist[bin >> 2], 1u << ((bin & 3) * 8));
+        }
         local = warp_sum(local);
         if (lane < kSamplerCtas)  // the same value in all lanes: lane c tells CTA c
             asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer_smem(&warp_sums[cta * (kClassesPerCta / 32) + warp], lane)), "f"(local) : "memory");
@@ -197,19 +212,8 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
         return;
     }
 
-    // ---- the entries that can matter, from the classes' largest ones ----
-    // As many entries reach F as classes' largest ones do: F = the lower end of the bin that holds the `want`th largest of these.
-    // Division by the total keeps the order but may join neighbours, so whoever reaches F / total as a probability is taken; the
-    // division is left out where t_i is further below F than its rounding.
     int inc, cnt;
-    auto count_down = [&]() {  // thread b holds bin 1023 - b of all CTAs: an inclusive scan counts the entries of that bin and all higher ones
-        cnt = 0;
-#pragma unroll
-        for (int z = 0; z < kSamplerCtas; ++z) {
-            int v;
-            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(peer_smem(&hist[kSamplerBins - 1 - tid], z)) : "memory");
-            cnt += v;
-        }
+    auto scan = [&]() {  // inc = the sum of cnt over this thread and those before it
         inc = cnt;
 #pragma unroll
         for (int m = 1; m < 32; m <<= 1) {
@@ -220,40 +224,85 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
         __syncthreads();
         inc += __reduce_add_sync(0xffffffffu, lane < warp ? scan_s[lane] : 0);
     };
+    auto count_down = [&]() {  // thread b holds bin 1023 - b of all CTAs: the scan counts the entries of that bin and all higher ones
+        cnt = 0;
+#pragma unroll
+        for (int z = 0; z < kSamplerCtas; ++z) {
+            int v;
+            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(peer_smem(&hist[kSamplerBins - 1 - tid], z)) : "memory");
+            cnt += v;
+        }
+        scan();
+    };
     const uint32_t n_list0 = peer_smem(&n_list, 0), list0 = peer_smem(list, 0);
     auto take = [&](uint64_t key) {
         int at;
         asm volatile("atom.relaxed.cluster.shared::cluster.add.s32 %0, [%1], 1;" : "=r"(at) : "r"(n_list0) : "memory");
         if (at < kSamplerCap) {
             asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(list0 + (uint32_t)at * 8), "l"(key) : "memory");
-        } else {
+        } else if (at == kSamplerCap) {  // one thread of the cluster tells all CTAs
             for (int z = 0; z < kSamplerCtas; ++z) asm volatile("st.shared::cluster.s32 [%0], 1;" ::"r"(peer_smem(&over_s, z)) : "memory");
         }
     };
+
+    // ---- the entries that can matter, from the classes' largest ones ----
+    // As many entries reach F as classes' largest ones do: F = the lower end of the bin that holds the `want`th largest of these.
+    // Division by the total keeps the order but may join neighbours, so whoever reaches F / total as a probability is taken; the
+    // division is left out where t_i is further below F than its rounding.
+    // Entries fall into classes as if by lot, so where c of the 1024 classes reach F, about -1024 ln(1 - c / 1024) entries do: the
+    // list's 2048 at c = 885.  Above kClassesListed (logits that are nearly all alike) the list is not tried.  us a draw over 128256 entries,
+    // top_k 50, with the radix select alone and so: 43.0 / 44.3 all equal, 36.9 / 38.9 with 2100 equal ones on top, 43.4 / 49.2 with 3224 of
+    // them in 224 classes (the list is tried and full), 32.8 / 30.7 with 2000, 18.4 / 14.4 normal ones about -20, 20.5 / 14.4 of deviation 2.5 at temperature 0.2.
+    bool listed = false;
     if (by_class) {
-        count_down();
-        if (inc >= p.want && inc - cnt < p.want) bin_s = kSamplerBins - 1 - tid;
+        uint32_t even = 0, odd = 0;  // of four bins: counts of the first and the third, of the second and the fourth
+#pragma unroll
+        for (int z = 0; z < kSamplerCtas; ++z) {
+            uint32_t v;
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_smem(&class_hist[kClassBinWords - 1 - tid], z)) : "memory");
+            even += v & 0x00ff00ffu;
+            odd += (v >> 8) & 0x00ff00ffu;
+        }
+        const int c[4] = {(int)(even & 0xffff), (int)(odd & 0xffff), (int)(even >> 16), (int)(odd >> 16)};
+        cnt = c[0] + c[1] + c[2] + c[3];
+        scan();
+        if (inc >= p.want && inc - cnt < p.want) {
+            int reach = inc - cnt, bin = 0;
+#pragma unroll
+            for (int j = 3; j >= 0; --j) {
+                if (reach < p.want) {
+                    reach += c[j];
+                    bin = 4 * (kClassBinWords - 1 - tid) + j;
+                }
+            }
+            bin_s = bin;
+            count_s = reach;
+        }
         __syncthreads();
+        listed = count_s <= kClassesListed;  // the same in all CTAs
     }
-    if (bin_s >= 0) {  // the same in all CTAs; else there are fewer classes than wanted entries
-        const float floor_t = class_bin_floor(bin_s), floor_p = __fdiv_rn(floor_t, total), near_t = floor_t * 0.999999f;
-#pragma unroll 4
-        for (int row = row0; row < rows; row += kRowsPerPass) {
-            const int i = row * kSamplerClasses + cls;
-            const float v = i < p.vocab ? t[(size_t)row * t_stride + col] : -1.0f;
-            if (v >= near_t) {
-                const float pr = __fdiv_rn(v, total);
-                if (pr >= floor_p) take(sample_key(pr, i));
+    if (listed) {
+        const float floor_t = class_bin_floor(bin_s), floor_p = __fdiv_rn(floor_t, total);
+        const float near_t = floor_p > 1e-30f ? floor_t * 0.999999f : 0.0f;  // a quotient with fewer bits joins more
+        for (int base = row0; base < rows; base += 4 * kRowsPerPass) {
+            if (*reinterpret_cast<volatile int *>(&over_s)) break;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = (base + j * kRowsPerPass) * kSamplerClasses + cls;
+                const float v = i < p.vocab ? t[(size_t)(base + j * kRowsPerPass) * t_stride + col] : -1.0f;
+                if (v >= near_t) {
+                    const float pr = __fdiv_rn(v, total);
+                    if (pr >= floor_p) take(sample_key(pr, i));
+                }
             }
         }
-    }
-    if (by_class) sampler_cluster_sync();
-    if (bin_s < 0 || over_s) {  // too many reach F: the general way.  The same in every thread of the cluster
-        if (by_class) {
-            if (tid == 0) n_list = 0;
-            hist[tid] = 0;
-            __syncthreads();
+        sampler_cluster_sync();
+        if (over_s) {
+            listed = false;
+            if (tid == 0) n_list = 0;  // a cluster barrier or more before the next entry is taken
         }
+    }
+    if (!listed) {  // the general way
         // ---- p_i, and a key prefix that enough entries reach ----
         for (int row = row0; row < rows; row += kRowsPerPass) {
             if (row * kSamplerClasses + cls >= p.vocab) break;
@@ -366,6 +415,8 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     const int token = (int)(0xffffffffu - (uint32_t)list[at]);
     p.token_out[0] = token;
     p.result[0] = 0;
+    p.result[1] = n;
+    p.result[2] = listed ? 1 : 0;
     if (p.pos && p.history) {
         const int where = p.pos[0];
         if (where >= 0 && where < p.history_len) p.history[where] = token;
