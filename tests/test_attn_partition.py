@@ -1,7 +1,6 @@
 """The tile shares of the batched decode attention (csrc/attn_decode.cu, balanced grid), restated on the host: group c
 of n_kv_heads CTAs takes tiles [c*Q, (c+1)*Q) of the 64-row tiles of all sequences numbered sequence by sequence, with
-Q = max(ceil(total / groups), split_len / 64, ceil(longest / n_splits)), and no less than the longest sequence where that has
-at most `whole` tiles (four where the engine chooses the split length, none where a caller has).  Checked for random mixes of lengths: every
+Q = max(ceil(total / groups), split_len / 64, ceil(longest / n_splits)).  Checked for random mixes of lengths: every
 tile is taken exactly once, a sequence is cut into at most n_splits + 1 pieces (the scratch holds n_splits + 1 slots
 per (sequence, KV head)), its pieces use the slots 0 .. n_used - 1 in order, and all of them agree on n_used."""
 import random
@@ -9,15 +8,13 @@ import random
 TILE = 64
 
 
-def partition(lens, groups, n_splits, split_len, whole=0):
+def partition(lens, groups, n_splits, split_len):
     tiles = [(l + TILE - 1) // TILE for l in lens]
     pre = [0]
     for t in tiles:
         pre.append(pre[-1] + t)
     total, longest = pre[-1], max(tiles)
     quota = max((total + groups - 1) // groups, max(max(split_len // TILE, 1), (longest + n_splits - 1) // n_splits))
-    if longest <= whole:
-        quota = max(quota, longest)
     pieces = []  # (group, seq, first row, end row, slot, n_used)
     for grp in range(groups):
         t, t_end = grp * quota, min((grp + 1) * quota, total)
@@ -34,8 +31,8 @@ def partition(lens, groups, n_splits, split_len, whole=0):
     return pieces
 
 
-def check(lens, groups, n_splits, split_len, whole):
-    pieces = partition(lens, groups, n_splits, split_len, whole)
+def check(lens, groups, n_splits, split_len):
+    pieces = partition(lens, groups, n_splits, split_len)
     for s, length in enumerate(lens):
         mine = sorted((p for p in pieces if p[1] == s), key=lambda p: p[2])
         assert mine, (s, lens)
@@ -53,14 +50,14 @@ def test_every_tile_once_and_pieces_fit_the_slots():
     rng = random.Random(7)
     for _ in range(400):
         n_seqs = rng.randint(2, 256)
-        max_len = rng.choice([1, 65, 200, 256, 257, 700, 4224, 8192])
+        max_len = rng.choice([1, 65, 700, 4224, 8192])
         lens = [rng.randint(1, max_len) for _ in range(n_seqs)]
         if rng.random() < 0.3:
             lens[rng.randrange(n_seqs)] = max_len
         split_len = rng.choice([32, 64, 128, 256, 1024])
         n_splits = max(1, (max(lens) + split_len - 1) // split_len)
         groups = rng.choice([1, 3, 55, 111, 444])
-        check(lens, groups, n_splits, split_len, rng.choice([0, 4]))
+        check(lens, groups, n_splits, split_len)
 
 
 def test_uniform_batch_of_the_benchmark():
@@ -68,11 +65,3 @@ def test_uniform_batch_of_the_benchmark():
     pieces = partition([1100] * 32, 55, 5, 256)
     assert max(p[3] - p[2] for p in pieces) <= 11 * TILE
     assert len({p[0] for p in pieces}) == 53   # 576 tiles / 11 per group
-    assert partition([1100] * 32, 55, 16, 128, 4) == pieces  # the engine's own split length: the even share is larger than either
-
-
-def test_short_sequences_of_the_engine():
-    # whole where the even share is smaller than a sequence, cut on the multiples of Q where it is larger
-    assert len(partition([200] * 5, 55, 4, 128, 4)) == 5 and len(partition([200] * 5, 55, 4, 128)) == 10
-    assert len(partition([256] * 13, 55, 4, 128, 4)) == 13
-    assert len(partition([208] * 96, 55, 4, 128, 4)) == 96 + 41  # quota 7
