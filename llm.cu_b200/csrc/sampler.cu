@@ -19,18 +19,18 @@
 //              that rounding may carry the prefix past the first top_k (see want_entries).  Whoever adds a class also keeps its
 //              largest t_i; as many entries as classes reach the `want`th largest of these, so the entries that do (usually not
 //              many more than wanted) go to CTA 0, which sorts them: one pass over the t_i without division or histogram.  Where
-//              nearly all classes or more than kSamplerCap entries do, or more than half as many entries as classes are wanted, a radix
-//              select over the 64-bit key (bits of p, then inverted index, so that keys are unique and equal p keep index order)
-//              finds a key prefix that between `want` and kSamplerCap entries reach.
+//              nearly all classes or more than kSamplerCap entries do, where more than half as many entries as classes are wanted or the
+//              vocabulary is small, a radix select over the 64-bit key (bits of p, then inverted index, so that keys are unique and
+//              equal p keep index order) finds a key prefix that between `want` and kSamplerCap entries reach.
 //   chain      the reference's statements on CTA 0: the running sums are one thread's, in the reference's order; the
 //              divisions between them are elementwise and use all threads.
 // Taking the entries one at a time by a block-wide argmax on a single CTA (every round: two barriers, and the owner's
-// rescan of its entries) took 495 us a draw at top_k 50 over 128256 entries; this form takes 14.4 us at any temperature (18.5 with the radix
-// select for all; 20 before short lists were ranked by counting and the running sums lost their load and branch per entry).
+// rescan of its entries) took 495 us a draw at top_k 50 over 128256 entries; this form takes 14.4 us (18.5 with the radix
+// select for all, whose time depends on how the logits are spread; 20 before short lists were ranked by counting and the running sums lost their load and branch per entry).
 // Different from the host code: the sum of the t_i is a tree over classes, not a loop in index order, and expf is CUDA's,
 // so probabilities can differ from the host's by a few FP32 ulps; the token differs only if u lies within that distance
 // of a boundary between two entries.
-#include <type_traits>
+#include <climits>
 
 #include "common.cuh"
 #include "../../include/llm_b200_synth.h"
@@ -47,7 +47,7 @@ constexpr int kSamplerCap = 2048;                                      // entrie
 constexpr int kSamplerSmemRows = 384;                                  // 192 KB of t_i per CTA: vocabularies up to 393216
 constexpr int kSamplerBins = 1024;
 constexpr int kClassBinWords = 1024;                                   // 4096 bins of the classes' largest t_i
-constexpr int kClassesListed = 880;  // classes whose largest entry reaches the floor, at most, for the list to be tried (see sample_kernel)
+constexpr int kClassesListed = 880;  // classes whose largest entry reaches the floor, at most, for the list to be tried (see the kernel)
 constexpr int kRankThreads = 4, kSamplerRankCap = kSamplerThreads / kRankThreads;  // up to 256 keys are ranked by counting
 
 struct SamplerParams {
@@ -106,8 +106,8 @@ __device__ __forceinline__ uint64_t sample_key(float pr, int i) {
 
 // Bins of the classes' largest t_i: 16 to an octave over all of FP32, so that the scale of the logits and the temperature do not
 // matter.  A CTA has 128 classes: a bin's count is a byte, four bins a word.
-__device__ __forceinline__ int class_bin(float t) { return (int)(__float_as_uint(t) >> 19); }
-__device__ __forceinline__ float class_bin_floor(int bin) { return __uint_as_float((uint32_t)bin << 19); }
+constexpr int kClassBinShift = 19;
+__device__ __forceinline__ int class_bin(float t) { return (int)(__float_as_uint(t) >> kClassBinShift); }
 
 // Index of the first entry whose running sum (in order, one rounding per entry) satisfies `hit`, -1 if none does; `run` =
 // the running sum up to it (or of all n).  No probability is negative, so a sum of eight is looked at only if its last
@@ -132,6 +132,10 @@ __device__ __forceinline__ int first_reaching(const float *v, int n, float &run,
     return -1;
 }
 
+// LOADS of a thread in flight at first: sixteen over 128256 entries take 2 us less than eight; a thread with fewer rows works through the
+// empty ones, 0.8 us over 8193 entries with sixteen instead of four.  One instantiation each, and one without the classes: a draw runs
+// through its code once, so code that it passes by costs too (0.1 to 0.2 us).
+template <bool BY_CLASS, int LOADS>
 __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerParams p) {
     extern __shared__ float t_smem[];               // [rows][128] t_i, then p_i, of this CTA's classes
     __shared__ float warp_sums[32];                 // of all CTAs
@@ -151,45 +155,36 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     pdl_launch_dependents();
     pdl_wait();
 
-    // The classes' largest entries lead to the wanted ones only where these are fewer than the classes, and it pays where a class has
-    // many (us a draw at 32768 / 65536 / 128256 entries, top_k 50: 11.0 / 12.6 / 18.5 without, 10.3 / 12.3 / 14.4 with it; over 4096 it lost 0.5).
-    const bool by_class = p.want <= kSamplerClasses / 2 && p.vocab > 8 * kSamplerClasses;
     // ---- t_i of this CTA's classes: thread = class cls, rows row0, row0 + 8, ... ----
     const int cls = (int)cta * kClassesPerCta + (tid & (kClassesPerCta - 1)), row0 = tid / kClassesPerCta;
     const int rows = (p.vocab + kSamplerClasses - 1) / kSamplerClasses;
     // element (row, class) of the vocabulary: t[row * t_stride + (class within the CTA)]
     float *t = p.in_smem ? t_smem : p.probs + (size_t)cta * kClassesPerCta;
     const int t_stride = p.in_smem ? kClassesPerCta : kSamplerClasses, col = tid & (kClassesPerCta - 1);
-    auto exponentials = [&](auto loads) {  // so many of a thread's loads in flight
-        constexpr int L = decltype(loads)::value;
-        for (int base = row0; base < rows; base += L * kRowsPerPass) {
-            __half x[L];
+    for (int base = row0; base < rows; base += LOADS * kRowsPerPass) {
+        __half x[LOADS];
 #pragma unroll
-            for (int j = 0; j < L; ++j) {
-                const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
-                x[j] = row < rows && i < p.vocab ? p.logits[i] : __half(0.0f);
-            }
-#pragma unroll
-            for (int j = 0; j < L; ++j) {
-                const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
-                if (row < rows && i < p.vocab) t[(size_t)row * t_stride + col] = expf(__fdiv_rn(__half2float(x[j]), p.temperature));
-            }
+        for (int j = 0; j < LOADS; ++j) {
+            const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
+            x[j] = row < rows && i < p.vocab ? p.logits[i] : __half(0.0f);
         }
-    };
-    // sixteen: eight took up to 2 us more over 128256 entries.  One where a thread has no second row: 18.9 us against 19.5 over 4096
-    // entries at top_k 500, 21.2 against 22.8 over 8192
-    if (rows <= kRowsPerPass) exponentials(std::integral_constant<int, 1>());
-    else exponentials(std::integral_constant<int, 16>());
+#pragma unroll
+        for (int j = 0; j < LOADS; ++j) {
+            const int row = base + j * kRowsPerPass, i = row * kSamplerClasses + cls;
+            if (row < rows && i < p.vocab) t[(size_t)row * t_stride + col] = expf(__fdiv_rn(__half2float(x[j]), p.temperature));
+        }
+    }
     hist[tid] = 0;
-    class_hist[tid] = 0;
+    if (BY_CLASS) class_hist[tid] = 0;
     if (tid == 0) {
         n_list = 0;
         over_s = 0;
     }
     __syncthreads();
     sampler_cluster_started_wait();
+    float most = 0.0f;  // of the class `tid` (of the CTA)
     if (tid < kClassesPerCta) {  // here col == tid
-        float local = 0.0f, most = 0.0f;
+        float local = 0.0f;
         const int n = cls < p.vocab ? (p.vocab - cls + kSamplerClasses - 1) / kSamplerClasses : 0;
 #pragma unroll 8
         for (int row = 0; row < n; ++row) {
@@ -197,7 +192,7 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
             local += v;
             most = fmaxf(most, v);
         }
-        if (n > 0 && by_class) {
+        if (BY_CLASS && n > 0) {
             const int bin = class_bin(most);
             atomicAdd(&class_hist[bin >> 2], 1u << ((bin & 3) * 8));
         }
@@ -249,12 +244,16 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     // As many entries reach F as classes' largest ones do: F = the lower end of the bin that holds the `want`th largest of these.
     // Division by the total keeps the order but may join neighbours, so whoever reaches F / total as a probability is taken; the
     // division is left out where t_i is further below F than its rounding.
-    // Entries fall into classes as if by lot, so where c of the 1024 classes reach F, about -1024 ln(1 - c / 1024) entries do: the
-    // list's 2048 at c = 885.  Above kClassesListed (logits that are nearly all alike) the list is not tried.  us a draw over 128256 entries,
-    // top_k 50, with the radix select alone and so: 43.0 / 44.3 all equal, 36.9 / 38.9 with 2100 equal ones on top, 43.4 / 49.2 with 3224 of
-    // them in 224 classes (the list is tried and full), 32.8 / 30.7 with 2000, 18.4 / 14.4 normal ones about -20, 20.5 / 14.4 of deviation 2.5 at temperature 0.2.
-    bool listed = false;
-    if (by_class) {
+    // Entries fall into classes as if by lot, so where c of the 1024 classes reach F, about -1024 ln(1 - c / 1024) entries do.  CTA 0 ranks
+    // up to 256 entries by counting (c = 226) and sorts more with a network of 512, 1024 (c = 403, 647) or 2048, 4 us and more each, so
+    // where the bin lets more classes pass than the wanted entries need, the next ten bits of its classes' largest are counted too
+    // (1.6 us).  Above kClassesListed (logits that are all alike; the list's 2048 entries are c = 885) the list is not tried.  us a
+    // draw, graph of 50, with the radix select alone / so, top_k 50: deviation 1.3 at temperature 0.7 over 32768 / 65536 / 128256 / 200000 entries
+    // 9.3 / 8.6, 11.7 / 10.5, 16.6 / 13.0, 22.1 / 16.8; over 128256 at temperature 0.1 18.0 / 12.5, about -20 16.5 / 12.8, deviation 0.05 21.3 / 14.7, 0.01 21.6 / 14.7,
+    // all equal 41.2 / 44.0, 20 not masked 46.6 / 48.6, 3224 equal ones on top in 224 classes (the list is tried and full) 37.4 / 44.8.
+    bool listed = false, finer = false;
+    uint32_t floor_bits = 0;
+    if (BY_CLASS) {
         uint32_t even = 0, odd = 0;  // of four bins: counts of the first and the third, of the second and the fourth
 #pragma unroll
         for (int z = 0; z < kSamplerCtas; ++z) {
@@ -267,22 +266,42 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
         cnt = c[0] + c[1] + c[2] + c[3];
         scan();
         if (inc >= p.want && inc - cnt < p.want) {
-            int reach = inc - cnt, bin = 0;
+            int reach = inc - cnt, bin = 0, above = 0;
 #pragma unroll
             for (int j = 3; j >= 0; --j) {
                 if (reach < p.want) {
+                    above = reach;
                     reach += c[j];
                     bin = 4 * (kClassBinWords - 1 - tid) + j;
                 }
             }
             bin_s = bin;
+            above_s = above;
             count_s = reach;
         }
         __syncthreads();
-        listed = count_s <= kClassesListed;  // the same in all CTAs
+        // all of this the same in all CTAs
+        floor_bits = (uint32_t)bin_s << kClassBinShift;
+        int classes = count_s;
+        if (bin_s > 0 && classes > (p.want <= 200 ? 220 : p.want <= 390 ? 400 : 640)) {
+            finer = true;
+            const int need = p.want - above_s, above = above_s;
+            if (tid < kClassesPerCta && class_bin(most) == bin_s) atomicAdd(&hist[(__float_as_uint(most) >> (kClassBinShift - 10)) & (kSamplerBins - 1)], 1);
+            sampler_cluster_sync();
+            count_down();
+            if (inc >= need && inc - cnt < need) {
+                bin_s = kSamplerBins - 1 - tid;
+                count_s = above + inc;
+            }
+            __syncthreads();
+            floor_bits |= (uint32_t)bin_s << (kClassBinShift - 10);
+            classes = count_s;
+            if (classes > kClassesListed) sampler_cluster_sync();  // every CTA has read the histograms
+        }
+        listed = classes <= kClassesListed;
     }
     if (listed) {
-        const float floor_t = class_bin_floor(bin_s), floor_p = __fdiv_rn(floor_t, total);
+        const float floor_t = __uint_as_float(floor_bits), floor_p = __fdiv_rn(floor_t, total);
         const float near_t = floor_p > 1e-30f ? floor_t * 0.999999f : 0.0f;  // a quotient with fewer bits joins more
         for (int base = row0; base < rows; base += 4 * kRowsPerPass) {
             if (*reinterpret_cast<volatile int *>(&over_s)) break;
@@ -303,6 +322,10 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
         }
     }
     if (!listed) {  // the general way
+        if (finer) {
+            hist[tid] = 0;
+            __syncthreads();
+        }
         // ---- p_i, and a key prefix that enough entries reach ----
         for (int row = row0; row < rows; row += kRowsPerPass) {
             if (row * kSamplerClasses + cls >= p.vocab) break;
@@ -423,6 +446,10 @@ __global__ void __launch_bounds__(kSamplerThreads) sample_kernel(const SamplerPa
     }
 }
 
+// The classes' largest entries lead to the wanted ones only where these are fewer than the classes, and it pays where a class has many: us a
+// draw at top_k 50 with the radix select / so 8.1 / 8.4 over 8193 entries, 8.5 / 8.7 over 16384, 9.1 / 9.0 over 20000, 9.3 / 8.6 over 32768.
+static bool sample_by_class(int vocab, int want) { return want <= kSamplerClasses / 2 && vocab >= 32 * kSamplerClasses; }
+
 }  // namespace llmb
 
 extern "C" size_t llmb_sample_scratch_bytes(int vocab) { return vocab > 0 ? (size_t)vocab * sizeof(float) + 256 : 0; }
@@ -459,9 +486,16 @@ extern "C" int llmb_sample_logits(const uint16_t *d_logits, int vocab, float tem
     const int rows = (vocab + kSamplerClasses - 1) / kSamplerClasses;
     p.in_smem = rows <= kSamplerSmemRows ? 1 : 0;
     const size_t smem = p.in_smem ? (size_t)rows * kClassesPerCta * sizeof(float) : 0;
-    static size_t attr_set[kMaxDevices] = {};
-    LLMB_CUDA_OK(ensure_dynamic_smem(sample_kernel, attr_set, smem));
-    LLMB_CUDA_OK(launch_pdl_cluster(sample_kernel, dim3(kSamplerCtas), dim3(kSamplerThreads), smem, static_cast<cudaStream_t>(stream_),
+    static size_t attr_set[2][3][kMaxDevices] = {};  // per instantiation and device
+    static const struct { void (*kernel)(const SamplerParams); int most_rows; } kernels[2][3] = {
+        {{sample_kernel<false, 1>, kRowsPerPass}, {sample_kernel<false, 4>, 4 * kRowsPerPass}, {sample_kernel<false, 16>, INT_MAX}},
+        {{nullptr, 0}, {sample_kernel<true, 4>, 4 * kRowsPerPass}, {sample_kernel<true, 16>, INT_MAX}}};
+    const int by_class = sample_by_class(vocab, p.want) ? 1 : 0;
+    int loads = 0;
+    while (rows > kernels[by_class][loads].most_rows) ++loads;
+    void (*kernel)(const SamplerParams) = kernels[by_class][loads].kernel;
+    LLMB_CUDA_OK(ensure_dynamic_smem(kernel, attr_set[by_class][loads], smem));
+    LLMB_CUDA_OK(launch_pdl_cluster(kernel, dim3(kSamplerCtas), dim3(kSamplerThreads), smem, static_cast<cudaStream_t>(stream_),
                                     use_pdl != 0, dim3(kSamplerCtas, 1, 1), p));
     return LLMB_OK;
 }
