@@ -237,7 +237,7 @@ __device__ __forceinline__ void finish_cols(const GemmParams &p, int row, int co
 
 // [rows][k] FP16 row-major as a 2-D tensor map with a 64 x box_rows box and 128-byte swizzle (gemm_tc.cu).  L2 fetches 256 bytes at a
 // time: the next K step of a row is needed next, and HBM gives more in longer runs (a stream of 128-row boxes from two CTAs per
-// SM 5.4 TB/s with 128 bytes, 5.9 with 256; batched steps of 5 x 333 / 32 x 1024 / 96 x 200 3.75 / 4.62 / 5.20 -> 3.54 / 4.43 / 5.09 ms).
+// SM 5.4 TB/s with 128 bytes, 5.9 with 256; batched steps of 5 x 333 / 32 x 1024 / 96 x 200 3.63 / 4.54 / 5.15 -> 3.43 / 4.39 / 5.08 ms).
 int make_map(CUtensorMap *map, const void *base, int rows, int k, int box_rows);
 
 // [d2][d1][d0] FP16 with strides of d1 and d2 in elements (d0 contiguous) as a 3-D tensor map, box 64 x box1 x box2 in

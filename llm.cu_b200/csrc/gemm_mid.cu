@@ -1,5 +1,5 @@
-// Projections of middling prompt blocks (129 to about 1000 rows at the 8B shape; not SwiGLU): C[M][N] = A[M][K] . B[N][K]^T where
-// the tiles are one wave: a CTA per tile and SM.  Same arithmetic as gemm_tc.cu.
+// Projections of middling prompt blocks (of the 8B shape 129 to 672 rows of QKV, to 896 of o_proj and down_proj; not SwiGLU):
+// C[M][N] = A[M][K] . B[N][K]^T where the tiles are one wave: a CTA per tile and SM.  Same arithmetic as gemm_tc.cu.
 //
 // The WEIGHTS are the 128-row operand of tcgen05.mma and the block's rows are its columns, as in gemm_smallm.cu, because the
 // number of columns can be any multiple of 16: with 128-row tiles of the block 517 rows are 640, and the 160 tiles of o_proj
@@ -7,11 +7,12 @@
 //
 // Bound: L2 to shared memory.  Per K step of 16 an SM loads (128 + nt) x 32 bytes, at 62 to 64 bytes a cycle, and the MMA takes
 // max(nt / 2, 32 + nt / 4) cycles (both measured): 64 + nt / 2 cycles a step, and no less than 120 with a stage of four steps, the
-// time of the waits, copies and MMAs of a stage.  So nt does not go below 96; where that leaves half of the SMs idle, K is cut in two
+// time of the waits, copies and MMAs of a stage.  So lower tiles than about 96 rows (M in ceil(M / 96) tiles, at the least 80 rows each)
+// gain nothing; where that leaves half of the SMs idle, K is cut in two
 // and the two CTAs of a tile are a cluster: each leaves the sums of half of the columns in its shared memory (the ring, free by
-// then) for the other, which adds them in slice order and finishes them.  Without slices, us at m = 200 / 384 / 517 rows (8B shape, from HBM) against
-// gemm_tc: QKV 45.1 / 47.0 / 55.7 -> 31.0 / 35.1 / 41.6, o_proj 32.9 / 33.7 / 36.8 -> 24.8 / 26.9 / 29.8, down_proj 65.7 / 96.0 / 101.8 -> 63.8 / 68.8 / 77.5
-// (launched one by one, 10 us of each are the launch).
+// then) for the other, which adds them in slice order and finishes them.  us at m = 200 / 384 / 517 rows (8B shape, weights from HBM, a graph of
+// launches) against gemm_tc: QKV 31.9 / 31.6 / 34.8 -> 24.0 / 29.2 / 32.5, o_proj 29.3 / 30.1 / 31.5 -> 19.3 / 22.3 / 28.7, down_proj 61.4 / 92.8 / 95.6 ->
+// 41.0 / 49.2 / 73.0.
 // The K of a CTA is summed in two accumulators, four up to 128 columns (all 512 columns of tensor memory), which the epilogue adds: tcgen05.mma
 // truncates where it adds to its accumulator, an error that grows with the length of the chain.
 //
@@ -265,9 +266,17 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 // Rows of a tile and slices of K where all tiles are one wave of at least 3/8 of the SMs; 0 rows where they are not.  Of the cuts of
 // the rows and the one or two slices the pair whose CTAs take least time, a step of 16 at max(121, 64 + nt / 2) cycles.  Prompts of 129 /
 // 200 / 256 tokens without slices 6.40 / 6.42 / 6.57 ms, with them 5.39 / 5.60 / 5.85.
+// Two slices from k = 2048 on (32 K steps): below, the exchange can cost more than the shorter K saves.  us with two slices / one,
+// n = 4096, m = 200: k = 512 10.5 / 11.4, 1024 11.5 / 13.6, 2048 14.0 / 18.0, 4096 18.6 / 26.0; m = 384: 11.9 / 10.4, 13.3 / 12.6, 16.2 / 16.7, 21.9 / 24.9.
+// 3/8 of the SMs keeps the cost honest where one slice would leave most of them idle: 300 x 2176 x 1024 in 3 cuts (51 CTAs) 13.3 us, in 4 11.9.
+// It only decides below k = 2048 (above, two slices double the CTAs), and there also leaves a few sizes to gemm_tc.cu that this kernel
+// would do faster (n 3200 to 3456 at up to 192 rows, 2176 and 2304 at 257 to 288: 160 x 3200 x 1024 19.1 us there, 12.0 here).
 // From 225 rows a tile on gemm_wide.cu is as fast or faster: prompts of 1000 / 1024 tokens (o_proj and down_proj in tiles of 256) 15.6 / 15.6 ->
-// 15.9 / 16.2 ms with this kernel.  Where gemm_tc.cu cuts K into three and more parts, its sums are in shorter chains than here: it
-// keeps those.
+// 15.9 / 16.2 ms with this kernel.  At 224 rows in one slice the kernel alone is slower than gemm_wide.cu and gemm_tc.cu (672 x 6144 x 4096
+// 36.9 us against 31.9, 896 x 4096 x 4096 36.3 against 33.4: its start, 7.5 us against 5, counts), but not behind another kernel whose end
+// hides that: prompts of 640 / 672 / 896 tokens take 11.0 / 11.9 / 14.5 ms either way.  For the same reason it is slower alone at
+// k below about 1200 (484 x 1920 x 192 9.3 us against 6.2); its four accumulators of up to 128 rows are the more exact there.
+// Where gemm_tc.cu cuts K into three and more parts, its sums are in shorter chains than here: it keeps those.
 static int mid_tile_rows(int m, int n, int k, int sms, int &splits) {
     const int w_tiles = (n + kBM - 1) / kBM;
     int best = 0, least = 0;

@@ -1153,9 +1153,10 @@ extern "C" int inference_continue(Llama3 *m, CudaCache *cache, int n_steps, int 
 // ---------------------------------------------------------------------------------------------
 namespace {
 
-// Cache rows per attention CTA where the caller has not said.  ms a step (8B) with 64 / 128 / 256 rows: 1 x 200 3.37 / 3.40 / 3.27 (fixed
-// splits; of several sequences those of up to 256 rows stay whole), 5 x 100 3.37 / 3.31 / 3.44, 5 x 333 3.59 / 3.46 / 3.59, 16 x 500
-// 3.79 / 3.76 / 3.88, 32 x 1024 4.42 / 4.39 / 4.43, 96 x 200 5.10 / 5.09 / 5.21.
+// Cache rows per attention CTA where the caller has not said.  ms a step (8B) with 64 / 128 / 256 rows, set by the caller: several sequences
+// 5 x 100 3.42 / 3.37 / 3.50, 5 x 333 3.61 / 3.50 / 3.61, 16 x 500 3.80 / 3.80 / 3.91; 2 x 600 128 / 256 rows 3.38 / 3.52, 4 x 400 3.47 / 3.61, 24 x 300 3.84 / 4.02;
+// no difference where the even share is larger than either (32 x 1024 4.5, 48 x 600 4.7, 96 x 200 5.1, 128 x 200 5.6: the same pieces).  A batch of
+// one (fixed splits): 200 rows 3.39 / 3.43 / 3.25, 300 3.45 / 3.46 / 3.43, 500 3.43 / 3.47 / 3.48, 1000 3.45 / 3.49 / 3.50, 1500 3.52 / 3.48 / 3.54.
 constexpr int kBatchWholeRows = 256;  // then also: no piece shorter than the longest sequence, if that has no more rows than this
 int batch_split_len(const Engine *e) { return e->bt_split_len > 0 ? e->bt_split_len : e->bt_seqs == 1 ? 256 : 128; }
 
