@@ -273,8 +273,8 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 // would do faster (n 3200 to 3456 at up to 192 rows, 2176 and 2304 at 257 to 288: 160 x 3200 x 1024 19.1 us there, 12.0 here).
 // From 225 rows a tile on gemm_wide.cu is as fast or faster: prompts of 1000 / 1024 tokens (o_proj and down_proj in tiles of 256) 15.6 / 15.6 ->
 // 15.9 / 16.2 ms with this kernel.  At 224 rows in one slice the kernel alone is slower than gemm_wide.cu and gemm_tc.cu (672 x 6144 x 4096
-// 36.9 us against 31.9, 896 x 4096 x 4096 36.3 against 33.4: its start, 7.5 us against 5, counts), but not behind another kernel whose end
-// hides that: prompts of 640 / 672 / 896 tokens take 11.0 / 11.9 / 14.5 ms either way.  For the same reason it is slower alone at
+// 36.9 us against 31.9, 896 x 4096 x 4096 36.3 against 33.4: the part that does not grow with K, 7.5 us against 5, counts), but not behind another kernel whose
+// end hides that: prompts of 640 / 672 / 896 tokens take 11.0 / 11.9 / 14.5 ms either way.  For the same reason it is slower alone at
 // k below about 1200 (484 x 1920 x 192 9.3 us against 6.2); its four accumulators of up to 128 rows are the more exact there.
 // Where gemm_tc.cu cuts K into three and more parts, its sums are in shorter chains than here: it keeps those.
 static int mid_tile_rows(int m, int n, int k, int sms, int &splits) {
